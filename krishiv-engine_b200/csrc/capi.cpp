@@ -295,6 +295,8 @@ static krv_status join_probe_impl(krv_join *j, const In *in, const ArrowSchema *
                 b = take_all(std::move(outs), j->spec().max_output_rows, j->pending);
             } else {
                 b = take_first(j->j->probe(inb), j->j->spec().max_output_rows, j->pending);
+                // the caller's device buffers are its own again when the call returns
+                if (Device && j->j->emitting()) KRV_CUDA(cudaStreamSynchronize(rt->stream));
             }
         } else {
             if (j->pending.empty()) krv::fail(KRV_INVALID_ARGUMENT, "no pending output and no input");

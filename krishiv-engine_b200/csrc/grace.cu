@@ -269,7 +269,8 @@ __global__ void __launch_bounds__(kGProbeThreads) grace_probe_kernel(const GPart
         bool live[kGRows];
         int64_t prow[kGRows];
         long long key[kGRows], bk[kGRows];
-        unsigned long long tag[kGRows], sl[kGRows];
+        uint32_t tag[kGRows];
+        unsigned long long sl[kGRows];
         uint64_t pos[kGRows];
         uint32_t cand[kGRows], cur[kGRows];
 #pragma unroll
@@ -279,14 +280,14 @@ __global__ void __launch_bounds__(kGProbeThreads) grace_probe_kernel(const GPart
             prow[u] = sp->prow0 + local;
             key[u] = live[u] ? out.pkey[prow[u]] : 0;
             const uint64_t g = finalize(hash_word((uint64_t)key[u]), seed);
-            tag[u] = g >> 32;
+            tag[u] = slot_tag(g);
             pos[u] = g & mask;
         }
 #pragma unroll
         for (int u = 0; u < kGRows; u++) sl[u] = live[u] ? __ldg(slots + pos[u]) : 0ull;
 #pragma unroll
         for (int u = 0; u < kGRows; u++) {
-            cand[u] = (sl[u] != 0 && (sl[u] >> 32) == tag[u]) ? (uint32_t)(sl[u] & 0xFFFFFFFFull) - 1u : kGNone;
+            cand[u] = sl[u] != 0 && slot_matches(sl[u], tag[u]) ? slot_row(sl[u]) : kGNone;
             bk[u] = cand[u] != kGNone ? __ldg(bkey + cand[u]) : 0;
         }
 #pragma unroll
@@ -302,8 +303,8 @@ __global__ void __launch_bounds__(kGProbeThreads) grace_probe_kernel(const GPart
             for (uint64_t probes = 1; probes <= mask; probes++) {
                 const unsigned long long s2 = __ldg(slots + q);
                 if (s2 == 0) break;
-                if ((s2 >> 32) == tag[u]) {
-                    const uint32_t o = (uint32_t)(s2 & 0xFFFFFFFFull) - 1u;
+                if (slot_matches(s2, tag[u])) {
+                    const uint32_t o = slot_row(s2);
                     if (__ldg(bkey + o) == key[u]) {
                         cur[u] = o;
                         break;

@@ -1,19 +1,22 @@
 // join.cu -- the hash join operator: build arena, open-addressing table over
-// the engine's key hash, warp-cooperative probe with warp-aggregated output
-// compaction fused with the payload gather, and the right/full join tails.
+// the engine's key hash, one probe kernel over row tiles whose output is
+// reserved per tile and written with the payload gather fused in, and the
+// right/full join tails.
 //
 // Reference: crates/krishiv-exec/src/join/ (HashJoin, join/mod.rs:1014;
 // BuildSink, join/build.rs; ProbeOp, join/probe.rs; JoinIndex,
 // crates/krishiv-exec/src/rows/index.rs).
 //
-// Table layout (one per join): `slots` is a power-of-two array of u64,
-// each (tag << 32) | (row + 1) with tag the top 32 bits of g = fin(h ^ seed)
-// and 0 = empty, probed linearly from g & mask; `next` chains the build rows
-// of one key newest-first (the reference's salted directory keeps a 16-bit
-// salt and row + 1 the same way, rows/index.rs:1-32, 211-283). A probe reads
-// a build row's key only when the 32-bit tag matches.
+// Table layout (one per join): `slots` is a power-of-two array of u64, each a
+// chained bit, 31 tag bits of g = fin(h ^ seed) and row + 1 (krv_device.cuh),
+// 0 = empty, probed linearly from g & mask; `next` chains the build rows of
+// one key newest-first (the reference's salted directory keeps a 16-bit salt
+// and row + 1 the same way, rows/index.rs:1-32, 211-283). A probe reads a
+// build row's key only when the tag matches, and its chain link only when the
+// slot says that the key has more rows.
 #include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "krv_device.cuh"
 #include "ops.h"
@@ -94,85 +97,145 @@ __device__ __forceinline__ bool eq_of(const KeysDev &a, int64_t i, const KeysDev
     return keys_eq(a, i, b, j);
 }
 
+// The table's insertion: kBuildRows rows per thread side by side, so that
+// their slot reads, compare-and-swaps and key compares (each a round trip to
+// L2) are in flight together.
+// ctr (zeroed): [0] distinct keys, [1] a NULL `=` key seen, [2] / [3] the
+// largest ~order(k) / order(k) of an int64 key (FAST), [4] indexed rows,
+// [5] status bits. The counts are reduced per CTA and the grid is a few CTAs
+// per SM: with one update per warp and counter, all on one cache line, the
+// updates took most of the kernel. Two rows per thread suit one int64 key
+// (four measured 10% slower), one row any other key (more code per row; two
+// rows measured 50% slower). krv_join_build_finish on B200, before -> after:
+// 1M unique keys 150 -> 89 us, 3M keys with duplicates 225 -> 130 us, 2M
+// (int64, int32) keys 140 -> 118 us.
+constexpr int kBuildThreads = 256;
+constexpr int kBuildRowsFast = 2, kBuildRowsAny = 1;
+constexpr unsigned long long kOrderBit = 1ull << 63;  // int64 order as unsigned order
 template <bool FAST>
-__global__ void __launch_bounds__(256) build_kernel(KeysDev keys, int64_t n, unsigned long long *slots,
-                                                    uint64_t mask, uint32_t *next, uint64_t seed,
-                                                    unsigned long long *ctr, uint32_t *status) {
-    // ctr: [0] distinct keys, [1] a NULL `=` key seen, [2] min / [3] max of an
-    // int64 key (FAST), [4] indexed rows.
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    unsigned long long heads = 0, rows = 0;
-    long long lo = LLONG_MAX, hi = LLONG_MIN;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-        uint32_t nx = kNone;
-        if (!matchable(keys, i)) {
-            next[i] = nx;
-            ctr[1] = 1;  // a NULL `=` key in the build (null-aware anti join)
-            continue;
+__global__ void __launch_bounds__(kBuildThreads) build_kernel(KeysDev keys, int64_t n, unsigned long long *slots,
+                                                              uint64_t mask, uint32_t *next, uint64_t seed,
+                                                              unsigned long long *ctr) {
+    constexpr int U = FAST ? kBuildRowsFast : kBuildRowsAny, kWarps = kBuildThreads / 32;
+    __shared__ unsigned long long s_red[4][kWarps];
+    unsigned long long heads = 0, rows = 0, lo = 0, hi = 0;
+    bool nulls = false, full = false;
+    const int64_t step = (int64_t)gridDim.x * kBuildThreads * U;
+    for (int64_t b0 = (int64_t)blockIdx.x * kBuildThreads * U; b0 < n; b0 += step) {
+        const int64_t i0 = b0 + threadIdx.x;
+        bool act[U];
+        uint32_t tag[U], nx[U];
+        uint64_t pos[U];
+        unsigned long long s[U], entry[U];
+        bool more = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t i = i0 + u * kBuildThreads;
+            act[u] = i < n && matchable(keys, i);
+            nulls = nulls || (i < n && !act[u]);
+            nx[u] = kNone;
+            tag[u] = 0;
+            pos[u] = 0;
+            entry[u] = 0;
+            if (!act[u]) continue;
+            more = true;
+            rows++;
+            if (FAST) {
+                const unsigned long long k = static_cast<const unsigned long long *>(keys.c[0].data)[i] ^ kOrderBit;
+                lo = ~k > lo ? ~k : lo;
+                hi = k > hi ? k : hi;
+            }
+            const uint64_t g = finalize(hash_of<FAST>(keys, i), seed);
+            tag[u] = slot_tag(g);
+            pos[u] = g & mask;
+            entry[u] = ((unsigned long long)tag[u] << 32) | (unsigned long long)(i + 1);
         }
-        rows++;
-        if (FAST) {
-            const long long k = static_cast<const long long *>(keys.c[0].data)[i];
-            lo = k < lo ? k : lo;
-            hi = k > hi ? k : hi;
-        }
-        const uint64_t g = finalize(hash_of<FAST>(keys, i), seed);
-        const unsigned long long entry = ((g >> 32) << 32) | (unsigned long long)(i + 1);
-        uint64_t pos = g & mask;
-        for (uint64_t probes = 0;; probes++) {
-            if (probes > mask) {
-                atomicOr(status, ST_CAPACITY);
+#pragma unroll
+        for (int u = 0; u < U; u++) s[u] = act[u] ? __ldcg(slots + pos[u]) : 0ull;
+        // every row is at a slot it has read: claim it when empty, else join
+        // its chain when the key is the row's, else go on to the next slot
+        for (uint64_t probes = 0; more; probes++) {
+            if (probes > 2 * mask + 2) {
+                full = true;  // more rows than slots: cannot happen below a load of 0.9
                 break;
             }
-            unsigned long long s = __ldcg(slots + pos);
-            if (s == 0) {
-                const unsigned long long old = atomicCAS(slots + pos, 0ull, entry);
-                if (old == 0) {
-                    heads++;
-                    break;
+            unsigned long long old[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) old[u] = act[u] && s[u] == 0 ? atomicCAS(slots + pos[u], 0ull, entry[u]) : 1ull;
+            bool eq[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (act[u] && s[u] == 0) {
+                    if (old[u] == 0) {
+                        heads++;
+                        act[u] = false;
+                    }
+                    s[u] = old[u];
                 }
-                s = old;
+                eq[u] = act[u] && slot_matches(s[u], tag[u]) &&
+                        eq_of<FAST>(keys, i0 + u * kBuildThreads, keys, slot_row(s[u]));
             }
-            if ((s >> 32) == (entry >> 32) && eq_of<FAST>(keys, i, keys, (int64_t)(s & 0xFFFFFFFFull) - 1)) {
-                // Same key: this row becomes the head, the old head its next.
-                const unsigned long long old = atomicExch(slots + pos, entry);
-                nx = (uint32_t)(old & 0xFFFFFFFFull) - 1u;
-                break;
+            more = false;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (!act[u]) continue;
+                if (eq[u]) {
+                    // Same key: this row becomes the head, the old head its next.
+                    nx[u] = slot_row(atomicExch(slots + pos[u], entry[u] | kSlotChained));
+                    act[u] = false;
+                    continue;
+                }
+                pos[u] = (pos[u] + 1) & mask;
+                s[u] = __ldcg(slots + pos[u]);
+                more = true;
             }
-            pos = (pos + 1) & mask;
         }
-        next[i] = nx;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i0 + u * kBuildThreads < n) next[i0 + u * kBuildThreads] = nx[u];
     }
-    // One atomic per warp and counter.
     for (int d = 16; d > 0; d >>= 1) {
-        heads += __shfl_xor_sync(0xFFFFFFFFu, heads, d);
-        rows += __shfl_xor_sync(0xFFFFFFFFu, rows, d);
-        const long long ol = __shfl_xor_sync(0xFFFFFFFFu, lo, d), oh = __shfl_xor_sync(0xFFFFFFFFu, hi, d);
-        lo = ol < lo ? ol : lo;
-        hi = oh > hi ? oh : hi;
+        heads += __shfl_xor_sync(kFull, heads, d);
+        rows += __shfl_xor_sync(kFull, rows, d);
+        lo = max(lo, __shfl_xor_sync(kFull, lo, d));
+        hi = max(hi, __shfl_xor_sync(kFull, hi, d));
     }
     if ((threadIdx.x & 31) == 0) {
-        if (heads) atomicAdd(ctr, heads);
-        if (rows) atomicAdd(ctr + 4, rows);
-        if (FAST && rows) {
-            atomicMin(reinterpret_cast<long long *>(ctr + 2), lo);
-            atomicMax(reinterpret_cast<long long *>(ctr + 3), hi);
-        }
+        s_red[0][threadIdx.x >> 5] = heads;
+        s_red[1][threadIdx.x >> 5] = rows;
+        s_red[2][threadIdx.x >> 5] = lo;
+        s_red[3][threadIdx.x >> 5] = hi;
     }
+    const bool any_null = __syncthreads_or(nulls), any_full = __syncthreads_or(full);
+    if (threadIdx.x) return;
+    for (int w = 1; w < kWarps; w++) {
+        heads += s_red[0][w];
+        rows += s_red[1][w];
+        lo = max(lo, s_red[2][w]);
+        hi = max(hi, s_red[3][w]);
+    }
+    if (heads) atomicAdd(ctr, heads);
+    if (rows) atomicAdd(ctr + 4, rows);
+    if (FAST && rows) {
+        atomicMax(ctr + 2, lo);
+        atomicMax(ctr + 3, hi);
+    }
+    if (any_null) ctr[1] = 1;  // a NULL `=` key in the build (null-aware anti join)
+    if (any_full) ctr[5] = ST_CAPACITY;
 }
 
 template <bool FAST>
 __device__ __forceinline__ uint32_t lookup(const KeysDev &pk, int64_t i, const KeysDev &bk,
                                            const unsigned long long *slots, uint64_t mask, uint64_t seed) {
     const uint64_t g = finalize(hash_of<FAST>(pk, i), seed);
-    const unsigned long long tag = g >> 32;
+    const uint32_t tag = slot_tag(g);
     uint64_t pos = g & mask;
     for (uint64_t probes = 0; probes <= mask; probes++) {
         const unsigned long long s = __ldg(slots + pos);
         if (s == 0) return kNone;
-        if ((s >> 32) == tag) {
-            const int64_t o = (int64_t)(s & 0xFFFFFFFFull) - 1;
-            if (eq_of<FAST>(pk, i, bk, o)) return (uint32_t)o;
+        if (slot_matches(s, tag)) {
+            const uint32_t o = slot_row(s);
+            if (eq_of<FAST>(pk, i, bk, o)) return o;
         }
         pos = (pos + 1) & mask;
     }
@@ -303,73 +366,64 @@ __device__ __forceinline__ void emit_round(const OutDev &out, bool want, unsigne
     }
 }
 
-// Allocates this round's output rows for the warp: returns the first row of
-// the round (same on every lane) and this lane's row.
-__device__ __forceinline__ unsigned long long round_alloc(unsigned long long *count, bool want,
-                                                          unsigned long long &pos) {
-    const unsigned ballot = __ballot_sync(kFull, want);
-    unsigned long long first = 0;
-    if (lane_id() == 0 && ballot) first = atomicAdd(count, (unsigned long long)__popc(ballot));
-    first = __shfl_sync(kFull, first, 0);
-    pos = first + __popc(ballot & lanemask_lt());
-    return first;
-}
-
-// Pairs: inner, left outer, right outer, full outer (join/probe.rs:266-502).
-template <bool FAST, bool FILT>
-__global__ void __launch_bounds__(256) probe_pairs_kernel(KeysDev pk, KeysDev bk, int64_t n,
-                                                          const unsigned long long *slots, uint64_t mask,
-                                                          const uint32_t *next, uint64_t seed, OutDev out,
-                                                          unsigned long long cap, unsigned long long *count,
-                                                          uint8_t *marks, int pads_probe, int single_match,
-                                                          uint32_t *status, unsigned long long *max_chain,
-                                                          FilterDev F) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        const bool live = i < n;
-        uint32_t cur = kNone;
-        if (live && matchable(pk, i)) cur = lookup<FAST>(pk, i, bk, slots, mask, seed);
-        if (FILT) cur = first_true(F, i, cur, next);
-        bool pad = live && cur == kNone && pads_probe;
-        unsigned chain = 0;
-        while (__any_sync(kFull, cur != kNone || pad)) {
-            const bool want = cur != kNone || pad;
-            unsigned long long pos;
-            const unsigned long long first = round_alloc(count, want, pos);
-            emit_round(out, want, pos, first, i, cur, cap);
-            if (cur != kNone) {
-                if (marks) marks[cur] = 1;
-                chain++;
-                cur = next[cur];
-                if (FILT) cur = first_true(F, i, cur, next);
-            } else {
-                pad = false;
-            }
-        }
-        if (single_match && chain > 1) atomicOr(status, ST_TOO_MANY);
-        if (chain > 1) atomicMax(max_chain, (unsigned long long)chain);
-    }
-}
-
-// Pairs of an inner or left outer join on one int64 `=` key over a build
-// side with unique keys, with no build marks: every probe row has at most one
-// output row, so the kernel has no chain walks and no per-row loops, and its
-// warps stay converged. Every lane resolves kFastRows probe rows at once
-// (their slot loads in flight together); the CTA scans its warps' counts in
-// shared memory and reserves its run of the output with one atomic per
-// kFastRows x 256 probe rows. Validity bits of nullable output columns are
-// set with one atomicOr per valid value.
+// ---- the probe ---------------------------------------------------------------------
+// Every probe that emits rows (inner, left / right / full outer, semi, anti;
+// join/probe.rs:266-502) takes two kernels and one host read between them:
+//  1. lookup_kernel finds each probe row's first build row (its head) and its
+//     number of output rows, writes both (4 or 8 B per row) and the sum of
+//     every tile of kTileRows rows; tile_scan_kernel turns the sums into every
+//     tile's first output row and tells the host the total;
+//  2. emit_kernel, into output columns of exactly that size, stages each
+//     tile's (probe row, build row) pairs in shared memory in output order,
+//     kWindow at a time, and writes them column by column: neighbouring
+//     threads write neighbouring output rows, so stores are coalesced, and a
+//     warp owns whole validity words.
+// The lookup is bound by the latency of its dependent random reads (slot,
+// build key, chain link), so it keeps few registers and many warps, with no
+// barrier or atomic between the reads; the emission is bound by the build
+// payload's random reads and the output's stores. One kernel for both
+// measured slower: it holds the registers of both phases and its warps wait at
+// the output reservation. On B200, the probe call, before (one output
+// reservation per warp and step, all on one counter) -> after: left outer of
+// 24M rows with 3M build rows of sparse keys, duplicates and NULLs 6.1 -> 0.99
+// ms (lookup 0.46, emission 0.46); semi join of 16M rows on (int64, int32)
+// 0.60 -> 0.43 ms; inner join of 10M rows over 1M dense keys 0.16 -> 0.15 ms.
 //
-// DIRECT: the build keys are also dense (their span at most a few times the
-// row count), and a direct index (key - lo -> build row) replaces the table:
-// one load per probe row instead of a slot load and a key compare.
-constexpr int kFastRows = 4;
-constexpr int kFastThreads = 256;
+// How a row finds its build rows:
+//  - kDirect: unique, dense int64 keys (`=`): an index of key - lo;
+//  - kUnique: no duplicate build keys: the slot's row is the only match;
+//  - kChains: the slot's row and its chain;
+//  - kRowsOnly: semi and anti joins: whether there is a match.
+enum Look : int { kDirect, kUnique, kChains, kRowsOnly };
+constexpr int kProbeThreads = 256;
+constexpr int kTileRows = 1024;
+constexpr int kRowsPerThread = 2;  // lookup: probe rows in flight per thread
+constexpr int kLookupBlocks = 6;   // resident lookup CTAs per SM
+constexpr int kEmitRows = kTileRows / kProbeThreads;
+constexpr int kEmitBlocks = 8;  // resident emission CTAs per SM
+constexpr int kWindow = 2048;  // staged pairs
 struct DirectDev {
     const uint32_t *row;  // build row of key lo + i, kNone where no row has it
     long long lo;
     unsigned long long span;  // hi - lo
+};
+struct ProbeDev {
+    KeysDev pk, bk;
+    int64_t n;
+    const unsigned long long *slots;
+    uint64_t mask;
+    const uint32_t *next;
+    uint64_t seed;
+    DirectDev dir;
+    uint8_t *marks;             // build rows that matched (null: not wanted)
+    int pad;                    // unmatched probe rows are emitted with a NULL build side
+    int single_match;
+    int kind;                   // kRowsOnly: 0 semi, 1 anti, 2 null-aware anti
+    int build_empty, build_has_null;
+    uint32_t *head;             // per row: its first build row, kNone; kRowsOnly: 0 an output row, kNone none
+    uint32_t *cnt;              // kChains: per row, its output rows
+    unsigned long long *tiles;  // per tile: its output rows, then (scanned) its first output row
+    uint32_t *status;           // single_match: ST_TOO_MANY
 };
 
 __global__ void direct_build_kernel(KeysDev bk, int64_t n, DirectDev d) {
@@ -381,144 +435,493 @@ __global__ void direct_build_kernel(KeysDev bk, int64_t n, DirectDev d) {
     }
 }
 
-template <bool DIRECT>
-__global__ void __launch_bounds__(kFastThreads) probe_fast_kernel(KeysDev pk, KeysDev bk, int64_t n,
-                                                                  const unsigned long long *slots, uint64_t mask,
-                                                                  uint64_t seed, DirectDev dir, OutDev out,
-                                                                  unsigned long long cap, unsigned long long *count,
-                                                                  int pad) {
-    constexpr int kWarps = kFastThreads / 32;
-    __shared__ unsigned s_warp[kWarps];
-    __shared__ unsigned long long s_base;
-    const long long *pkeys = static_cast<const long long *>(pk.c[0].data);
-    const long long *bkeys = static_cast<const long long *>(bk.c[0].data);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t tile = (int64_t)kFastThreads * kFastRows;
-    for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
-        int64_t row[kFastRows];
-        uint32_t head[kFastRows];
-        long long key[kFastRows];
-        uint64_t pos[kFastRows];
-        unsigned long long tag[kFastRows], slot[kFastRows];
-        bool live[kFastRows];
+// NK key columns known to the compiler (0: a loop over any number), so that
+// the loads of all columns and rows are in flight together.
+template <int NK>
+__device__ __forceinline__ void hash_rows_of(const KeysDev &K, int64_t r0, const bool (&look)[kRowsPerThread],
+                                             uint64_t (&h)[kRowsPerThread]) {
+    constexpr int U = kRowsPerThread, M = NK ? NK : 1;
+    const int n = NK ? NK : K.n;
 #pragma unroll
-        for (int u = 0; u < kFastRows; u++) {
-            row[u] = base + (int64_t)u * kFastThreads + threadIdx.x;
-            live[u] = row[u] < n && key_valid(pk.c[0], row[u]);
-            key[u] = live[u] ? pkeys[row[u]] : 0;
-            if (DIRECT) continue;
-            const uint64_t g = finalize(hash_word((uint64_t)key[u]), seed);
-            tag[u] = g >> 32;
-            pos[u] = g & mask;
-        }
-        if (DIRECT) {
+    for (int u = 0; u < U; u++) h[u] = 0;  // fold(SEEDLESS = 0, MIX)
+    for (int c0 = 0; c0 < n; c0 += M) {
+        uint64_t w0[M][U], w1[M][U];
+        bool v[M][U];
 #pragma unroll
-            for (int u = 0; u < kFastRows; u++) {
-                const unsigned long long off = (unsigned long long)key[u] - (unsigned long long)dir.lo;
-                head[u] = live[u] && off <= dir.span ? __ldg(dir.row + off) : kNone;
+        for (int c = 0; c < M; c++)
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                w0[c][u] = w1[c][u] = 0;
+                v[c][u] = look[u] && key_valid(K.c[c0 + c], r0 + u * kProbeThreads);
+                if (v[c][u]) key_words(K.c[c0 + c], r0 + u * kProbeThreads, w0[c][u], w1[c][u]);
             }
-        }
 #pragma unroll
-        for (int u = 0; u < kFastRows; u++) slot[u] = !DIRECT && live[u] ? __ldg(slots + pos[u]) : 0ull;
+        for (int c = 0; c < M; c++)
 #pragma unroll
-        for (int u = 0; u < kFastRows; u++) {
-            if (DIRECT) break;
-            head[u] = kNone;
-            if (!live[u]) continue;
-            unsigned long long sl = slot[u];
-            uint64_t p = pos[u];
-            for (uint64_t probes = 0; probes <= mask && sl != 0; probes++) {
-                if ((sl >> 32) == tag[u]) {
-                    const uint32_t o = (uint32_t)(sl & 0xFFFFFFFFull) - 1u;
-                    if (__ldg(bkeys + o) == key[u]) {
-                        head[u] = o;
-                        break;
-                    }
+            for (int u = 0; u < U; u++) {
+                if (v[c][u]) {
+                    h[u] = mix(h[u], w0[c][u]);
+                    if (K.c[c0 + c].width == 16) h[u] = mix(h[u], w1[c][u]);
+                } else if ((K.null_safe >> (c0 + c)) & 1u) {
+                    h[u] = mix(h[u], kNullHash);
                 }
-                p = (p + 1) & mask;
-                sl = __ldg(slots + p);
+            }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) h[u] = fold(h[u], kFinish);
+}
+
+// Whether the thread's probe rows and build rows cand[u] have equal keys (false
+// where cand[u] is kNone), all rows' loads in flight together.
+template <int NK>
+__device__ __forceinline__ void keys_equal(const ProbeDev &A, int64_t r0, const uint32_t (&cand)[kRowsPerThread],
+                                           bool (&eq)[kRowsPerThread]) {
+    constexpr int U = kRowsPerThread, M = NK ? NK : 1;
+    const int n = NK ? NK : A.pk.n;
+#pragma unroll
+    for (int u = 0; u < U; u++) eq[u] = cand[u] != kNone;
+    for (int c0 = 0; c0 < n; c0 += M) {
+        uint64_t b0[M][U], b1[M][U];
+        bool bv[M][U];
+#pragma unroll
+        for (int c = 0; c < M; c++)
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                b0[c][u] = b1[c][u] = 0;
+                bv[c][u] = cand[u] != kNone && key_valid(A.bk.c[c0 + c], cand[u]);
+                if (bv[c][u]) key_words(A.bk.c[c0 + c], cand[u], b0[c][u], b1[c][u]);
+            }
+#pragma unroll
+        for (int c = 0; c < M; c++)
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (!eq[u]) continue;
+                uint64_t p0 = 0, p1 = 0;
+                const bool pv = key_valid(A.pk.c[c0 + c], r0 + u * kProbeThreads);
+                if (pv) key_words(A.pk.c[c0 + c], r0 + u * kProbeThreads, p0, p1);
+                eq[u] = pv == bv[c][u] && p0 == b0[c][u] && p1 == b1[c][u];
+            }
+    }
+}
+
+// The build rows that head the chains of rows r0 + u * kProbeThreads
+// (kNone: no match; rows with look[u] false are not looked up), and whether
+// each chain has more than its head. KEY: 1 one int64 `=` key, 2 two key
+// columns, 0 any keys.
+template <int KEY>
+__device__ __forceinline__ void find_heads(const ProbeDev &A, int64_t r0, const bool (&look)[kRowsPerThread],
+                                           uint32_t (&head)[kRowsPerThread], bool (&chained)[kRowsPerThread]) {
+    constexpr int U = kRowsPerThread;
+    constexpr bool FAST = KEY == 1;
+    uint64_t h[U];
+    long long key[U];
+    const long long *bkeys = static_cast<const long long *>(A.bk.c[0].data);
+    if (FAST) {
+        const long long *pkeys = static_cast<const long long *>(A.pk.c[0].data);
+#pragma unroll
+        for (int u = 0; u < U; u++) key[u] = look[u] ? pkeys[r0 + u * kProbeThreads] : 0;
+#pragma unroll
+        for (int u = 0; u < U; u++) h[u] = hash_word((uint64_t)key[u]);
+    } else {
+        hash_rows_of<KEY>(A.pk, r0, look, h);
+    }
+    uint32_t tag[U];
+    uint64_t pos[U];
+    unsigned long long sl[U];
+    bool more = false;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint64_t g = finalize(h[u], A.seed);
+        tag[u] = slot_tag(g);
+        pos[u] = g & A.mask;
+        sl[u] = look[u] ? __ldg(A.slots + pos[u]) : 0ull;
+        head[u] = kNone;
+        chained[u] = false;
+        more = more || look[u];
+    }
+    // Every row steps to a slot of its tag or to an empty one (sl is 0 then),
+    // the rows of a thread side by side; then the keys are compared once. A
+    // tag names another key once in 2^31 times: such a row steps on.
+    for (uint64_t round = 0; more && round <= A.mask; round++) {
+        bool step = true;
+        for (uint64_t probes = 0; step && probes <= A.mask; probes++) {
+            step = false;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (sl[u] == 0 || slot_matches(sl[u], tag[u])) continue;
+                pos[u] = (pos[u] + 1) & A.mask;
+                sl[u] = __ldg(A.slots + pos[u]);
+                step = true;
             }
         }
-        bool emit[kFastRows];
-        unsigned mine = 0;
+        uint32_t cand[U];
+        bool eq[U];
 #pragma unroll
-        for (int u = 0; u < kFastRows; u++) {
-            emit[u] = row[u] < n && (head[u] != kNone || pad);
-            mine += emit[u];
-        }
-        unsigned incl = mine;
+        for (int u = 0; u < U; u++) cand[u] = sl[u] != 0 ? slot_row(sl[u]) : kNone;
+        if (FAST) {
+            long long bkey[U];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned y = __shfl_up_sync(kFull, incl, d);
-            if (lane >= d) incl += y;
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned acc = 0;
-            for (int w = 0; w < kWarps; w++) {
-                const unsigned c = s_warp[w];
-                s_warp[w] = acc;
-                acc += c;
-            }
-            s_base = acc ? atomicAdd(count, (unsigned long long)acc) : 0ull;
-        }
-        __syncthreads();
-        unsigned long long at = s_base + s_warp[warp] + (incl - mine);
-        __syncthreads();  // s_warp and s_base are rewritten by the next tile
+            for (int u = 0; u < U; u++) bkey[u] = cand[u] != kNone ? __ldg(bkeys + cand[u]) : 0;
 #pragma unroll
-        for (int u = 0; u < kFastRows; u++) {
-            if (!emit[u]) continue;
-            const unsigned long long a = at++;
-            if (a >= cap) continue;
-            const uint32_t b = head[u];
-            for (int k = 0; k < out.n; k++) {
-                const OutColDev &c = out.c[k];
-                bool v = false;
-                if (c.side == 3) {
-                    static_cast<long long *>(c.dst)[a] = row[u];
-                } else if (c.side == 4) {
-                    static_cast<long long *>(c.dst)[a] = b != kNone ? (long long)b : -1;
-                } else if (c.side == 0) {
-                    copy_value(c.dst, c.src, (int64_t)a, row[u], c.width);
-                    v = bit_get(c.src_valid, c.src_voff, row[u]);
-                } else if (b != kNone) {
-                    copy_value(c.dst, c.src, (int64_t)a, b, c.width);
-                    v = bit_get(c.src_valid, c.src_voff, b);
-                } else {
-                    zero_value(c.dst, (int64_t)a, c.width);
-                }
-                if (c.dst_valid && v) atomicOr(c.dst_valid + (a >> 5), 1u << (a & 31));
+            for (int u = 0; u < U; u++) eq[u] = cand[u] != kNone && bkey[u] == key[u];
+        } else {
+            keys_equal<KEY>(A, r0, cand, eq);
+        }
+        more = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (eq[u]) {
+                head[u] = cand[u];
+                chained[u] = (sl[u] & kSlotChained) != 0;
+                sl[u] = 0;
+            } else if (sl[u] != 0) {
+                pos[u] = (pos[u] + 1) & A.mask;
+                sl[u] = __ldg(A.slots + pos[u]);
+                more = true;
             }
         }
     }
 }
 
-// Probe rows once: semi, anti, null-aware anti (join/mod.rs:27-34).
-// kind 0 semi, 1 anti, 2 null-aware anti.
-template <bool FAST, bool FILT>
-__global__ void __launch_bounds__(256) probe_rows_kernel(KeysDev pk, KeysDev bk, int64_t n,
-                                                         const unsigned long long *slots, uint64_t mask,
-                                                         uint64_t seed, OutDev out, unsigned long long cap,
-                                                         unsigned long long *count, int kind, int build_empty,
-                                                         int build_has_null, const uint32_t *next, FilterDev F) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        const bool live = i < n;
-        bool ok = false;
-        if (live) {
-            const bool m = matchable(pk, i);
-            uint32_t c = m && !build_empty ? lookup<FAST>(pk, i, bk, slots, mask, seed) : kNone;
-            if (FILT) c = first_true(F, i, c, next);
-            const bool hit = c != kNone;
-            if (kind == 0) ok = hit;
-            else if (kind == 1) ok = !hit;
-            else ok = build_empty || (!build_has_null && m && !hit);
+template <int KEY, bool FILT, int LOOK>
+__global__ void __launch_bounds__(kProbeThreads, kLookupBlocks) lookup_kernel(ProbeDev A, FilterDev F) {
+    constexpr int U = kRowsPerThread, kWarps = kProbeThreads / 32;
+    __shared__ unsigned long long s_warp[kWarps];
+    const int64_t base = (int64_t)blockIdx.x * kTileRows;
+    unsigned long long total = 0;
+#pragma unroll 1
+    for (int step = 0; step < kTileRows / (kProbeThreads * U); step++) {
+        const int64_t r0 = base + step * (kProbeThreads * U) + threadIdx.x;
+        bool look[U], chained[U];
+        uint32_t cur[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t r = r0 + u * kProbeThreads;
+            look[u] = r < A.n && !A.build_empty && (KEY == 1 ? key_valid(A.pk.c[0], r) : matchable(A.pk, r));
+            cur[u] = kNone;
         }
-        unsigned long long pos;
-        const unsigned long long first = round_alloc(count, ok, pos);
-        emit_round(out, ok, pos, first, i, kNone, cap);
+        if (LOOK == kDirect) {
+            long long key[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                key[u] = look[u] ? static_cast<const long long *>(A.pk.c[0].data)[r0 + u * kProbeThreads] : 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const unsigned long long off = (unsigned long long)key[u] - (unsigned long long)A.dir.lo;
+                if (look[u] && off <= A.dir.span) cur[u] = __ldg(A.dir.row + off);
+            }
+        } else {
+            find_heads<KEY>(A, r0, look, cur, chained);
+        }
+        if (FILT)
+#pragma unroll
+            for (int u = 0; u < U; u++) cur[u] = first_true(F, r0 + u * kProbeThreads, cur[u], A.next);
+        uint32_t cnt[U];
+        if (LOOK == kChains) {
+            // the chains of all rows walked together
+            uint32_t w[U];
+            bool more = false;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                cnt[u] = cur[u] != kNone ? 1 : 0;
+                if (A.marks && cur[u] != kNone) A.marks[cur[u]] = 1;
+                w[u] = cur[u] != kNone && chained[u] ? cur[u] : kNone;
+                more = more || w[u] != kNone;
+            }
+            while (more) {
+                more = false;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (w[u] == kNone) continue;
+                    w[u] = __ldg(A.next + w[u]);
+                    if (FILT) w[u] = first_true(F, r0 + u * kProbeThreads, w[u], A.next);
+                    if (w[u] == kNone) continue;
+                    if (A.marks) A.marks[w[u]] = 1;
+                    cnt[u]++;
+                    more = true;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (A.single_match && cnt[u] > 1) atomicOr(A.status, ST_TOO_MANY);
+                if (cnt[u] == 0 && A.pad && r0 + u * kProbeThreads < A.n) cnt[u] = 1;
+            }
+        } else if (LOOK == kRowsOnly) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const bool hit = cur[u] != kNone;
+                bool ok = hit;
+                if (A.kind == 1) ok = !hit;
+                if (A.kind == 2) ok = A.build_empty || (!A.build_has_null && look[u] && !hit);
+                cnt[u] = ok && r0 + u * kProbeThreads < A.n ? 1 : 0;
+                cur[u] = cnt[u] ? 0u : kNone;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (A.marks && cur[u] != kNone) A.marks[cur[u]] = 1;
+                cnt[u] = cur[u] != kNone || (A.pad && r0 + u * kProbeThreads < A.n) ? 1 : 0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t r = r0 + u * kProbeThreads;
+            total += cnt[u];
+            if (r >= A.n) continue;
+            if (A.head) A.head[r] = cur[u];
+            if (LOOK == kChains && A.cnt) A.cnt[r] = cnt[u];
+        }
+    }
+    if (!A.tiles) return;  // only the marks are wanted (right semi / anti)
+    for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(kFull, total, d);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kWarps; w++) total += s_warp[w];
+        A.tiles[blockIdx.x] = total;
+    }
+}
+
+// Every tile's first output row (an exclusive scan of the tiles' rows, in
+// place); out[0] (mapped host memory): all rows, out[1]: the status word.
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(unsigned long long *tiles, int64_t n,
+                                                                 const uint32_t *status, volatile unsigned long long *out) {
+    __shared__ unsigned long long s_warp[kScanThreads / 32], s_run;
+    constexpr int kPer = 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long run = 0;
+    for (int64_t t0 = 0; t0 < n; t0 += kScanThreads * kPer) {
+        unsigned long long v[kPer], mine = 0;
+        const int64_t i0 = t0 + (int64_t)threadIdx.x * kPer;
+        if (i0 + kPer <= n) {
+#pragma unroll
+            for (int j = 0; j < kPer; j += 2) {
+                const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(tiles + i0 + j);
+                v[j] = x.x, v[j + 1] = x.y;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < kPer; j++) v[j] = i0 + j < n ? tiles[i0 + j] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; j++) mine += v[j];
+        unsigned long long incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, incl, d);
+            if (lane >= d) incl += y;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned long long w = s_warp[lane];
+            unsigned long long wi = w;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned long long y = __shfl_up_sync(kFull, wi, d);
+                if (lane >= d) wi += y;
+            }
+            s_warp[lane] = wi - w;
+            if (lane == 31) s_run = wi;
+        }
+        __syncthreads();
+        unsigned long long at = run + s_warp[warp] + incl - mine;
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            if (i0 + j < n) tiles[i0 + j] = at;
+            at += v[j];
+        }
+        run += s_run;
+        __syncthreads();  // s_warp and s_run are rewritten by the next chunk
+    }
+    if (threadIdx.x == 0) {
+        out[0] = run;
+        out[1] = status ? *status : 0u;
+    }
+}
+
+// What emit_kernel reads of the lookup.
+struct EmitDev {
+    int64_t row0, rows;  // the probe rows of this launch (head and cnt start at row0)
+    const uint32_t *head;
+    const uint32_t *cnt;
+    const unsigned long long *tiles;  // of the tiles from row0 on
+    const uint32_t *next;
+    int pad;
+};
+
+// One output column of a window's m pairs (output rows first .. first + m),
+// by the whole CTA: four pairs' loads, then their stores. `rows`: the pairs'
+// rows of the column's side (kNone: NULL). With validity words a warp starts
+// at a multiple of 32 output rows and owns whole words but the window's ends.
+template <class T, class R>
+__device__ __forceinline__ void emit_column(const OutColDev &c, const R *rows, int64_t base, unsigned long long first, int m) {
+    constexpr int V = 4;
+    const T *src = static_cast<const T *>(c.src) + (c.side == 0 ? base : 0);
+    T *dst = static_cast<T *>(c.dst) + first;
+    if (!c.dst_valid) {
+        for (int q0 = threadIdx.x; q0 < m; q0 += V * kProbeThreads) {
+            T v[V];
+#pragma unroll
+            for (int j = 0; j < V; j++) {
+                const int q = q0 + j * kProbeThreads;
+                v[j] = T{};
+                if (q >= m) continue;
+                const uint32_t r = rows[q];
+                if (sizeof(R) == 2 || r != kNone) v[j] = src[r];
+            }
+#pragma unroll
+            for (int j = 0; j < V; j++)
+                if (q0 + j * kProbeThreads < m) dst[q0 + j * kProbeThreads] = v[j];
+        }
+        return;
+    }
+    const int64_t voff = c.src_voff + (c.side == 0 ? base : 0);
+    for (int q0 = (int)threadIdx.x - (int)(first & 31); q0 - (int)threadIdx.x < m; q0 += kProbeThreads) {
+        const uint32_t r = (unsigned)q0 < (unsigned)m ? (uint32_t)rows[q0] : kNone;
+        const bool some = (unsigned)q0 < (unsigned)m && (sizeof(R) == 2 || r != kNone);
+        if ((unsigned)q0 < (unsigned)m) dst[q0] = some ? src[r] : T{};
+        const unsigned w = __ballot_sync(kFull, some && bit_get(c.src_valid, voff, r));
+        if (w && lane_id() == (unsigned)(__ffs(w) - 1)) {
+            const int first_lane = q0 - (int)lane_id();  // the word's first pair
+            uint32_t *p = c.dst_valid + ((unsigned long long)((long long)first + q0) >> 5);
+            if (first_lane >= 0 && first_lane + 32 <= m) *p = w;
+            else atomicOr(p, w);  // a word shared with the next window or tile (zeroed before)
+        }
+    }
+}
+template <class R>
+__device__ __forceinline__ void emit_by_width(const OutColDev &c, const R *rows, int64_t base, unsigned long long first, int m) {
+    if (c.width == 8) emit_column<uint64_t>(c, rows, base, first, m);
+    else if (c.width == 4) emit_column<uint32_t>(c, rows, base, first, m);
+    else if (c.width == 16) emit_column<uint4>(c, rows, base, first, m);
+    else emit_column<uint8_t>(c, rows, base, first, m);
+}
+
+template <bool FILT, int LOOK>
+__global__ void __launch_bounds__(kProbeThreads, kEmitBlocks) emit_kernel(EmitDev E, OutDev out, FilterDev F) {
+    constexpr int U = kEmitRows, kWarps = kProbeThreads / 32;
+    // a tile's output rows: at most one per probe row, or chains of any length
+    using Sum = std::conditional_t<LOOK == kChains, unsigned long long, uint32_t>;
+    static_assert(U == 4, "heads are read four at a time");
+    __shared__ Sum s_warp[kWarps];
+    __shared__ uint32_t s_brow[kWindow];
+    __shared__ uint16_t s_prow[kWindow];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t t0 = (int64_t)blockIdx.x * kTileRows;
+    const int64_t base = E.row0 + t0;  // the tile's first probe row
+    const int64_t l0 = t0 + threadIdx.x * U;
+    // neighbouring rows per thread: output order is probe order
+    const unsigned long long run = E.tiles[blockIdx.x];
+    uint32_t cur[U], cnt[U];
+    if (l0 + U <= E.rows) {
+        const uint4 h = *reinterpret_cast<const uint4 *>(E.head + l0);
+        cur[0] = h.x, cur[1] = h.y, cur[2] = h.z, cur[3] = h.w;
+        if (LOOK == kChains) {
+            const uint4 n = *reinterpret_cast<const uint4 *>(E.cnt + l0);
+            cnt[0] = n.x, cnt[1] = n.y, cnt[2] = n.z, cnt[3] = n.w;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            cur[u] = l0 + u < E.rows ? E.head[l0 + u] : kNone;
+            if (LOOK == kChains) cnt[u] = l0 + u < E.rows ? E.cnt[l0 + u] : 0;
+        }
+    }
+    Sum mine = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        if (LOOK != kChains) cnt[u] = cur[u] != kNone || (E.pad && l0 + u < E.rows) ? 1 : 0;
+        if (LOOK == kRowsOnly) cur[u] = kNone;
+        mine += cnt[u];
+    }
+    Sum incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const Sum y = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    Sum total = 0, before = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        const Sum c = s_warp[w];
+        before += w < warp ? c : 0;
+        total += c;
+    }
+    // staged pairs, a window of the tile's output at a time
+    Sum at = before + (incl - mine);
+    int ru = 0;  // this thread's row being staged
+    uint32_t left = cnt[0], b = cur[0];
+    for (Sum w0 = 0; w0 < total; w0 += kWindow) {
+        const unsigned m = total - w0 < kWindow ? (unsigned)(total - w0) : (unsigned)kWindow;
+        if (LOOK == kChains && total <= kWindow) {
+            // the chains of the thread's rows side by side: each step is a
+            // dependent random read
+            uint32_t off[U], r[U];
+            bool more = true;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                off[u] = (uint32_t)at;
+                at += cnt[u];
+                r[u] = cur[u];
+            }
+            for (uint32_t k = 0; more; k++) {
+                more = false;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (k >= cnt[u]) continue;
+                    s_prow[off[u] + k] = (uint16_t)(threadIdx.x * U + u);
+                    s_brow[off[u] + k] = r[u];
+                    if (k + 1 >= cnt[u]) continue;
+                    r[u] = __ldg(E.next + r[u]);
+                    if (FILT) r[u] = first_true(F, base + threadIdx.x * U + u, r[u], E.next);
+                    more = true;
+                }
+            }
+        } else if (LOOK == kChains) {
+            while (at < w0 + m) {
+                while (left == 0 && ru < U - 1) {
+                    ru++;
+#pragma unroll
+                    for (int u = 1; u < U; u++)
+                        if (u == ru) left = cnt[u], b = cur[u];
+                }
+                if (left == 0) break;  // every row of this thread is staged
+                s_prow[at - w0] = (uint16_t)(threadIdx.x * U + ru);
+                s_brow[at - w0] = b;
+                at++;
+                if (--left) {
+                    b = __ldg(E.next + b);
+                    if (FILT) b = first_true(F, base + threadIdx.x * U + ru, b, E.next);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (!cnt[u]) continue;
+                s_prow[at] = (uint16_t)(threadIdx.x * U + u);
+                s_brow[at] = cur[u];
+                at++;
+            }
+        }
+        __syncthreads();
+        const unsigned long long first = run + w0;
+        for (int k = 0; k < out.n; k++) {
+            const OutColDev c = out.c[k];
+            if (c.side == 0) {
+                emit_by_width(c, s_prow, base, first, (int)m);
+            } else if (c.side == 1) {
+                emit_by_width(c, s_brow, base, first, (int)m);
+            } else {  // the row index itself (3 probe, 4 build)
+                for (unsigned q = threadIdx.x; q < m; q += kProbeThreads)
+                    static_cast<long long *>(c.dst)[first + q] =
+                        c.side == 3 ? (long long)(base + s_prow[q]) : s_brow[q] != kNone ? (long long)s_brow[q] : -1ll;
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -541,6 +944,18 @@ __global__ void __launch_bounds__(256) probe_exists_kernel(KeysDev pk, KeysDev b
         const unsigned word = __ballot_sync(kFull, hit);
         if (lane_id() == 0 && (i < n)) exists[i >> 5] = word;
     }
+}
+
+// Allocates this round's output rows for the warp: returns the first row of
+// the round (same on every lane) and this lane's row.
+__device__ __forceinline__ unsigned long long round_alloc(unsigned long long *count, bool want,
+                                                          unsigned long long &pos) {
+    const unsigned ballot = __ballot_sync(kFull, want);
+    unsigned long long first = 0;
+    if (lane_id() == 0 && ballot) first = atomicAdd(count, (unsigned long long)__popc(ballot));
+    first = __shfl_sync(kFull, first, 0);
+    pos = first + __popc(ballot & lanemask_lt());
+    return first;
 }
 
 // Build rows by their marks once the probe side is done (emit_build,
@@ -612,7 +1027,9 @@ void hash_rows(Runtime *rt, const DevBatch &b, const int32_t *cols, int n, const
     check_launch("hash_rows_kernel");
 }
 
-static bool fast_keys(const KeysDev &k) { return k.n == 1 && k.c[0].width == 8 && !k.c[0].is_float; }
+// One int64 `=` key: hashed and compared as its value (a `<=>` key's NULL is a
+// key of its own, which the general code tells from every value).
+static bool fast_keys(const KeysDev &k) { return k.n == 1 && k.c[0].width == 8 && !k.c[0].is_float && !k.null_safe; }
 
 HashJoin::HashJoin(Runtime *rt, const krv_join_spec &spec) : rt_(rt), spec_(spec) {
     if (spec.n_keys < 1 || spec.n_keys > KRV_MAX_KEYS) fail(KRV_INVALID_ARGUMENT, "join needs 1..4 keys");
@@ -659,15 +1076,19 @@ void HashJoin::append_arena(const DevBatch &b) {
             const size_t w = t.var() ? 8 : (size_t)t.width();
             const size_t bytes = t.id == Type::Bool ? (size_t)ceil_div(cap, 8) : (size_t)cap * w;
             auto nd = std::make_shared<DBuf>(rt_, bytes);
-            auto nv = std::make_shared<DBuf>(rt_, (size_t)ceil_div(cap, 32) * 4 + 8);
-            zero(rt_, nv->get(), nv->bytes());
+            std::shared_ptr<DBuf> nv;
+            if (arena_valid_[i]) {
+                nv = std::make_shared<DBuf>(rt_, (size_t)ceil_div(cap, 32) * 4 + 8);
+                zero(rt_, nv->get(), nv->bytes());
+            }
             std::shared_ptr<DBuf> nl;
             if (t.var()) nl = std::make_shared<DBuf>(rt_, (size_t)cap * 4);
             if (build_rows_) {
                 const size_t old = t.id == Type::Bool ? (size_t)ceil_div(build_rows_, 8) : (size_t)build_rows_ * w;
                 KRV_CUDA(cudaMemcpyAsync(nd->get(), arena_data_[i]->get(), old, cudaMemcpyDeviceToDevice, rt_->stream));
-                KRV_CUDA(cudaMemcpyAsync(nv->get(), arena_valid_[i]->get(), (size_t)ceil_div(build_rows_, 8),
-                                         cudaMemcpyDeviceToDevice, rt_->stream));
+                if (nv)
+                    KRV_CUDA(cudaMemcpyAsync(nv->get(), arena_valid_[i]->get(), (size_t)ceil_div(build_rows_, 8),
+                                             cudaMemcpyDeviceToDevice, rt_->stream));
                 if (nl)
                     KRV_CUDA(cudaMemcpyAsync(nl->get(), arena_var_[i].lens->get(), (size_t)build_rows_ * 4,
                                              cudaMemcpyDeviceToDevice, rt_->stream));
@@ -694,7 +1115,13 @@ void HashJoin::append_arena(const DevBatch &b) {
             KRV_CUDA(cudaMemcpyAsync(arena_data_[i]->as<uint8_t>() + build_rows_ * w, c.data, (size_t)b.rows * w,
                                      cudaMemcpyDeviceToDevice, rt_->stream));
         }
-        append_bits(rt_, c.valid, c.valid_off, b.rows, arena_valid_[i]->as<uint8_t>(), build_rows_);
+        // a column keeps a bitmap from its first batch with one on
+        if (c.valid && !arena_valid_[i]) {
+            arena_valid_[i] = std::make_shared<DBuf>(rt_, (size_t)ceil_div(arena_cap_, 32) * 4 + 8);
+            zero(rt_, arena_valid_[i]->get(), arena_valid_[i]->bytes());
+            set_bits(rt_, arena_valid_[i]->as<uint8_t>(), 0, build_rows_);
+        }
+        if (arena_valid_[i]) append_bits(rt_, c.valid, c.valid_off, b.rows, arena_valid_[i]->as<uint8_t>(), build_rows_);
     }
     build_rows_ = need;
 }
@@ -736,7 +1163,7 @@ VarSrc HashJoin::var_src(int side, int col, const DevBatch *probe) const {
     v.starts = a.starts->as<long long>();
     v.lens = a.lens->as<int32_t>();
     v.bytes = a.heap ? a.heap->as<uint8_t>() : nullptr;
-    v.valid = arena_cols_[col].nullable ? arena_valid_[col]->as<uint8_t>() : nullptr;
+    v.valid = arena_cols_[col].nullable && arena_valid_[col] ? arena_valid_[col]->as<uint8_t>() : nullptr;
     return v;
 }
 
@@ -962,15 +1389,11 @@ void HashJoin::build_finish() {
     const uint64_t want = (uint64_t)std::ceil((double)std::max<int64_t>(build_rows_, 1) / spec_.max_load);
     const uint64_t slots = std::max<uint64_t>(1024, next_pow2(want));
     mask_ = slots - 1;
-    slots_ = DBuf(rt_, slots * 8);
-    zero(rt_, slots_.get(), slots * 8);
+    // the slots and, after them, the build's counters: one clearing
+    slots_ = DBuf(rt_, slots * 8 + 64);
+    zero(rt_, slots_.get(), slots * 8 + 64);
     next_ = DBuf(rt_, (size_t)std::max<int64_t>(build_rows_, 1) * 4);
-    counters_dev_ = DBuf(rt_, 64);
-    {
-        // [0] keys, [1] NULL seen, [2] min, [3] max, [4] indexed rows, [6] longest chain
-        const unsigned long long init[8] = {0, 0, (unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MIN, 0, 0, 0, 0};
-        KRV_CUDA(cudaMemcpyAsync(counters_dev_.get(), init, 64, cudaMemcpyHostToDevice, rt_->stream));
-    }
+    unsigned long long *ctr = slots_.as<unsigned long long>() + slots;
     const int jt = spec_.join_type;
     const bool preserved = jt == KRV_JOIN_RIGHT_SEMI || jt == KRV_JOIN_RIGHT_ANTI || jt == KRV_JOIN_RIGHT_OUTER ||
                            jt == KRV_JOIN_FULL_OUTER;
@@ -978,33 +1401,31 @@ void HashJoin::build_finish() {
         marks_ = DBuf(rt_, (size_t)std::max<int64_t>(build_rows_, 1));
         zero(rt_, marks_.get(), marks_.bytes());
     }
-    clear_status(rt_);
+    unsigned long long host_ctr[8] = {};
     if (build_rows_ > 0) {
         if (arena_.cols.empty()) fail(KRV_INVALID_ARGUMENT, "build batches without columns");
         KeysDev k = keys_of(arena_, spec_.build_keys, spec_.n_keys, spec_.null_safe);
-        const int threads = 256;
-        const int grid = grid_for(rt_, build_rows_, threads, 8);
-        auto *ctr = counters_dev_.as<unsigned long long>();
+        const int grid = grid_for(rt_, ceil_div(build_rows_, fast_keys(k) ? kBuildRowsFast : kBuildRowsAny), kBuildThreads,
+                                  fast_keys(k) ? 8 : 16);
         if (fast_keys(k))
-            build_kernel<true><<<grid, threads, 0, rt_->stream>>>(k, build_rows_, slots_.as<unsigned long long>(), mask_,
-                                                                 next_.as<uint32_t>(), spec_.seed, ctr, status_word(rt_));
+            build_kernel<true><<<grid, kBuildThreads, 0, rt_->stream>>>(k, build_rows_, slots_.as<unsigned long long>(),
+                                                                       mask_, next_.as<uint32_t>(), spec_.seed, ctr);
         else
-            build_kernel<false><<<grid, threads, 0, rt_->stream>>>(k, build_rows_, slots_.as<unsigned long long>(), mask_,
-                                                                  next_.as<uint32_t>(), spec_.seed, ctr, status_word(rt_));
+            build_kernel<false><<<grid, kBuildThreads, 0, rt_->stream>>>(k, build_rows_, slots_.as<unsigned long long>(),
+                                                                        mask_, next_.as<uint32_t>(), spec_.seed, ctr);
         rt_->launches++;
         check_launch("build_kernel");
+        read_device(rt_, ctr, 64, host_ctr);
+        if (host_ctr[5] & ST_CAPACITY) fail(KRV_INTERNAL, "join table full");
     }
-    unsigned long long host_ctr[8];
-    KRV_CUDA(cudaMemcpyAsync(host_ctr, counters_dev_.get(), 64, cudaMemcpyDeviceToHost, rt_->stream));
-    const uint32_t st = take_status(rt_);  // synchronizes: host_ctr is ready too
-    if (st & ST_CAPACITY) fail(KRV_INTERNAL, "join table full");
     counters_.build_rows = build_rows_;
     counters_.build_keys = (int64_t)host_ctr[0];
     counters_.table_slots = (int64_t)slots;
     any_null_build_ = host_ctr[1] != 0;
     indexed_rows_ = (int64_t)host_ctr[4];
-    key_lo_ = (long long)host_ctr[2];
-    key_hi_ = (long long)host_ctr[3];
+    // without rows: lo > hi
+    key_lo_ = indexed_rows_ ? (long long)(~host_ctr[2] ^ kOrderBit) : LLONG_MAX;
+    key_hi_ = indexed_rows_ ? (long long)(host_ctr[3] ^ kOrderBit) : LLONG_MIN;
     // Unique, dense int64 keys (a span of at most 4 values per row): a direct
     // index, 4 bytes per key value, for the probe of inner and left outer joins.
     direct_.reset();
@@ -1033,8 +1454,8 @@ void HashJoin::build_finish() {
             // The build already counted the kept rows, the distinct keys and
             // their range: the filter builder needs no pass of its own unless
             // an exact form may apply.
-            KeyStats ks{(int64_t)host_ctr[4], (int64_t)host_ctr[0], (long long)host_ctr[2], (long long)host_ctr[3]};
-            filter_ = build_key_filter(rt_, o, key, &ks);
+            KeyStats ks{(int64_t)host_ctr[4], (int64_t)host_ctr[0], key_lo_, key_hi_};
+            filter_ = build_key_filter(rt_, o, key, spec_.null_safe[0] ? nullptr : &ks);
         }
     }
 }
@@ -1060,6 +1481,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     const DevBatch &in = coded_ ? coded_in : outer_in;
     const int jt = spec_.join_type;
     const int64_t n = in.rows;
+    emitting_ = false;
     counters_.probe_rows += n;
     if (probe_types_.empty()) {
         for (const DevCol &c : in.cols) {
@@ -1082,25 +1504,70 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
         fail(KRV_INVALID_ARGUMENT, "has_residual_filter is set but no filter was given (krv_join_set_filter)");
     const bool filt = residual_set_;
     const FilterDev fd = filt ? filter_dev(in) : FilterDev{};
-    auto launch_pairs = [&](bool fast_, bool filt_, int grid_, int threads_, const KeysDev &pk_, const KeysDev &bk_,
-                            int64_t n_, const OutDev &od_, unsigned long long cap_, unsigned long long *count_,
-                            uint8_t *marks_p, int pad_, int single_, unsigned long long *mc_, const FilterDev &fd_) {
-        const auto *sl = slots_.as<unsigned long long>();
-        const uint32_t *nx = next_.as<uint32_t>();
-        uint32_t *st = status_word(rt_);
-        if (fast_ && filt_)
-            probe_pairs_kernel<true, true><<<grid_, threads_, 0, rt_->stream>>>(
-                pk_, bk_, n_, sl, mask_, nx, spec_.seed, od_, cap_, count_, marks_p, pad_, single_, st, mc_, fd_);
-        else if (fast_)
-            probe_pairs_kernel<true, false><<<grid_, threads_, 0, rt_->stream>>>(
-                pk_, bk_, n_, sl, mask_, nx, spec_.seed, od_, cap_, count_, marks_p, pad_, single_, st, mc_, fd_);
-        else if (filt_)
-            probe_pairs_kernel<false, true><<<grid_, threads_, 0, rt_->stream>>>(
-                pk_, bk_, n_, sl, mask_, nx, spec_.seed, od_, cap_, count_, marks_p, pad_, single_, st, mc_, fd_);
-        else
-            probe_pairs_kernel<false, false><<<grid_, threads_, 0, rt_->stream>>>(
-                pk_, bk_, n_, sl, mask_, nx, spec_.seed, od_, cap_, count_, marks_p, pad_, single_, st, mc_, fd_);
+    // The lookup over rows [row0, row0 + rows) (row0 a multiple of kTileRows).
+    auto launch_lookup = [&](int look, int64_t row0, int64_t rows, uint32_t *head, uint32_t *cnt,
+                             unsigned long long *tiles, uint8_t *marks, int pad, int kind, uint32_t *status) {
+        if (rows == 0) return;
+        ProbeDev A{};
+        A.pk = pk;
+        for (int k = 0; k < pk.n; k++) {
+            A.pk.c[k].data = static_cast<const uint8_t *>(pk.c[k].data) + row0 * pk.c[k].width;
+            A.pk.c[k].voff += row0;
+        }
+        A.bk = bk;
+        A.n = rows;
+        A.slots = slots_.as<unsigned long long>();
+        A.mask = mask_;
+        A.next = next_.as<uint32_t>();
+        A.seed = spec_.seed;
+        A.dir = DirectDev{direct_.as<uint32_t>(), key_lo_, direct_span_};
+        A.marks = marks;
+        A.pad = pad;
+        A.single_match = spec_.single_match;
+        A.kind = kind;
+        A.build_empty = build_rows_ == 0;
+        A.build_has_null = any_null_build_;
+        A.head = head;
+        A.cnt = cnt;
+        A.tiles = tiles;
+        A.status = status;
+        FilterDev f = fd;  // its probe columns from row0 on
+        for (int t = 0; t < f.n; t++)
+            for (FilterOpDev *o : {&f.t[t].l, &f.t[t].r})
+                if (o->side == 0) {
+                    o->data = static_cast<const uint8_t *>(o->data) + row0 * o->width;
+                    o->voff += row0;
+                }
+        const int grid = (int)ceil_div(rows, kTileRows);
+        auto go = [&](auto kernel) { kernel<<<grid, kProbeThreads, 0, rt_->stream>>>(A, f); };
+        auto by_keys = [&](auto l) {
+            constexpr int L = decltype(l)::value;
+            if (fast && filt) go(lookup_kernel<1, true, L>);
+            else if (fast) go(lookup_kernel<1, false, L>);
+            else if (filt) go(lookup_kernel<0, true, L>);
+            else if (pk.n == 2) go(lookup_kernel<2, false, L>);
+            else go(lookup_kernel<0, false, L>);
+        };
+        if (look == kDirect) go(lookup_kernel<1, false, kDirect>);
+        else if (look == kUnique) by_keys(std::integral_constant<int, kUnique>{});
+        else if (look == kChains) by_keys(std::integral_constant<int, kChains>{});
+        else by_keys(std::integral_constant<int, kRowsOnly>{});
+        rt_->launches++;
+        check_launch("lookup_kernel");
     };
+    auto launch_emit = [&](int look, const EmitDev &E, const OutDev &od) {
+        if (E.rows == 0 || od.n == 0) return;
+        const int grid = (int)ceil_div(E.rows, kTileRows);
+        if (look == kChains && filt) emit_kernel<true, kChains><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
+        else if (look == kChains) emit_kernel<false, kChains><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
+        else if (look == kRowsOnly) emit_kernel<false, kRowsOnly><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
+        else emit_kernel<false, kUnique><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
+        rt_->launches++;
+        check_launch("emit_kernel");
+    };
+    // unique build keys: at most one output row per probe row
+    const bool unique_keys = build_rows_ > 0 && counters_.build_keys == indexed_rows_;
+    const int look = !unique_keys ? kChains : fast && !filt && direct_.get() ? kDirect : kUnique;
     const auto pcols = projection(spec_.n_probe_out, spec_.probe_out, (int)in.cols.size());
     const auto bcols = projection(spec_.n_build_out, spec_.build_out, (int)arena_cols_.size());
     const int threads = 256;
@@ -1157,15 +1624,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     if (!pairs && (jt == KRV_JOIN_RIGHT_SEMI || jt == KRV_JOIN_RIGHT_ANTI)) {
         // Probe only marks build rows; output comes at finish.
         if (n > 0 && build_rows_ > 0) {
-            OutDev od{};
-            od.n = 0;
-            DBuf cnt(rt_, 8);
-            zero(rt_, cnt.get(), 8);
-            auto *mc = counters_dev_.as<unsigned long long>() + 6;
-            launch_pairs(fast, filt, grid, threads, pk, bk, n, od, 0, cnt.as<unsigned long long>(), marks_.as<uint8_t>(), 0,
-                         0, mc, fd);
-            rt_->launches++;
-            check_launch("probe_pairs_kernel");
+            launch_lookup(look, 0, n, nullptr, nullptr, nullptr, marks_.as<uint8_t>(), 0, 0, nullptr);
         }
         // Nothing is emitted by this batch: an empty batch of the output shape.
         DevBatch empty;
@@ -1175,140 +1634,137 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
 
     const bool build_nullable = jt == KRV_JOIN_LEFT_OUTER || jt == KRV_JOIN_FULL_OUTER;
     const bool probe_nullable = jt == KRV_JOIN_RIGHT_OUTER || jt == KRV_JOIN_FULL_OUTER;
-    // The output's size is known only after the kernel. Unique build keys
-    // give at most one row per probe row; otherwise there is room for the
-    // rows that the earlier batches' output ratio predicts (before any, the
-    // build's mean rows per key), 5% more, and a batch with more output runs
-    // again with room for all of it.
-    unsigned long long cap = (unsigned long long)std::max<int64_t>(n, 1);
-    const bool unique_keys = build_rows_ > 0 && counters_.build_keys == indexed_rows_;
-    if (pairs && !unique_keys && n > 0) {
-        const int64_t seen = counters_.probe_rows - n;
-        double ratio = seen > 0 ? (double)counters_.output_rows / (double)seen
-                       : counters_.build_keys > 0 ? (double)indexed_rows_ / (double)counters_.build_keys : 1.0;
-        if (jt == KRV_JOIN_LEFT_OUTER || jt == KRV_JOIN_FULL_OUTER) ratio = std::max(ratio, 1.0);
-        cap = std::max<unsigned long long>(1, (unsigned long long)((double)n * ratio * 1.05) + 1024);
+    const bool pads = jt == KRV_JOIN_LEFT_OUTER || jt == KRV_JOIN_FULL_OUTER;
+    const int kind = jt == KRV_JOIN_LEFT_SEMI ? 0 : jt == KRV_JOIN_LEFT_ANTI ? 1 : 2;
+    const int how = pairs ? look : kRowsOnly;
+    const bool none = n == 0 || (pairs && build_rows_ == 0 && !pads);  // no output rows
+    uint8_t *marks = marks_.get() ? marks_.as<uint8_t>() : nullptr;
+    const int64_t ntiles = ceil_div(n, (int64_t)kTileRows);
+    DBuf head, cnt, tiles, status;
+    int64_t chunk = n;  // rows looked up and emitted together
+    if (!none) {
+        if (spec_.single_match) {
+            status = DBuf(rt_, 8);
+            zero(rt_, status.get(), 8);
+        }
+        tiles = DBuf(rt_, (size_t)ntiles * 8);
+        try {
+            head = DBuf(rt_, (size_t)n * 4);
+            if (how == kChains) cnt = DBuf(rt_, (size_t)n * 4);
+        } catch (const Error &e) {
+            if (e.code != KRV_NEED_MEMORY) throw;
+            // No room to keep every row's lookup: count now, and look up
+            // again, a chunk at a time, when the rows are emitted.
+            head = DBuf();
+            chunk = std::min<int64_t>(n, 64 * kTileRows);
+        }
+        const bool kept = head.get() != nullptr;
+        launch_lookup(how, 0, n, kept ? head.as<uint32_t>() : nullptr, kept && how == kChains ? cnt.as<uint32_t>() : nullptr,
+                      tiles.as<unsigned long long>(), pairs ? marks : nullptr, pads && pairs, kind, status.as<uint32_t>());
+        tile_scan_kernel<<<1, kScanThreads, 0, rt_->stream>>>(
+            tiles.as<unsigned long long>(), ntiles, status.as<uint32_t>(),
+            reinterpret_cast<volatile unsigned long long *>(static_cast<uint8_t *>(rt_->status_host_dev) + 64));
+        rt_->launches++;
+        check_launch("tile_scan_kernel");
+        if (!kept) {
+            head = DBuf(rt_, (size_t)chunk * 4);
+            if (how == kChains) cnt = DBuf(rt_, (size_t)chunk * 4);
+        }
     }
-    DBuf cnt(rt_, 8);
-    for (int attempt = 0; attempt < 4; attempt++) {
+    auto total = [&]() -> int64_t {  // waits for the scan
+        if (none) return 0;
+        KRV_CUDA(cudaStreamSynchronize(rt_->stream));
+        volatile unsigned long long *seen =
+            reinterpret_cast<volatile unsigned long long *>(static_cast<uint8_t *>(rt_->status_host) + 64);
+        if (seen[1] & ST_TOO_MANY)
+            fail(KRV_TOO_MANY_ROWS, "SCALAR_SUBQUERY_TOO_MANY_ROWS: a probe row matched more than one build row");
+        return (int64_t)seen[0];
+    };
+    // The output columns for m rows, and the kernel that fills them.
+    std::vector<VarOut> vars;  // string columns, gathered once the row indexes are known
+    DBuf idx[2];
+    auto emit = [&](int64_t m) {
         out = DevBatch{};
+        vars.clear();
         OutDev od{};
-        std::vector<VarOut> vars;  // string columns, gathered once the row indexes are known
+        EmitDev E{};
+        auto column = [&](const DevCol &s, const DType &type, const std::string &name, const uint8_t *src_valid, int side,
+                          int col, bool nullable) {
+            if (type.var()) {
+                DevCol meta;
+                meta.type = type;
+                meta.name = name;
+                meta.nullable = nullable;
+                vars.push_back(VarOut{(int)out.cols.size(), side, col});
+                out.cols.push_back(meta);
+                return;
+            }
+            DevCol d = make_col(rt_, type, m, nullable, name);
+            if (d.valid) zero(rt_, const_cast<uint8_t *>(d.valid), d.hold_valid->bytes());
+            od.c[od.n++] = OutColDev{s.data, src_valid, s.valid_off, const_cast<void *>(d.data), (uint32_t *)d.valid,
+                                     type.width(), side};
+            out.cols.push_back(d);
+        };
         for (int pc : pcols) {
             const DevCol &s = in.cols[pc];
             if (s.type.id == Type::Bool) fail(KRV_UNSUPPORTED, "boolean probe payload columns");
-            const bool nullable = s.nullable || s.valid || probe_nullable;
-            if (s.type.var()) {
-                DevCol m;
-                m.type = s.type;
-                m.name = s.name;
-                m.nullable = nullable;
-                vars.push_back(VarOut{(int)out.cols.size(), 0, pc});
-                out.cols.push_back(m);
-                continue;
-            }
-            DevCol d = make_col(rt_, s.type, (int64_t)cap, nullable, s.name);
-            if (d.valid) zero(rt_, const_cast<uint8_t *>(d.valid), d.hold_valid->bytes());
-            od.c[od.n++] = OutColDev{s.data, s.valid, s.valid_off, const_cast<void *>(d.data),
-                                     (uint32_t *)d.valid, s.type.width(), 0};
-            out.cols.push_back(d);
+            column(s, s.type, s.name, s.valid, 0, pc, s.nullable || s.valid || probe_nullable);
         }
-        if (pairs) {
+        if (pairs)
             for (int bc : bcols) {
-                const DevCol &s = arena_.cols.empty() ? DevCol{} : arena_.cols[bc];
+                const DevCol s = arena_.cols.empty() ? DevCol{} : arena_.cols[bc];
                 const DevCol &meta = arena_cols_[bc];
-                const bool nullable = meta.nullable || build_nullable;
-                if (meta.type.var()) {
-                    DevCol m;
-                    m.type = meta.type;
-                    m.name = meta.name;
-                    m.nullable = nullable;
-                    vars.push_back(VarOut{(int)out.cols.size(), 1, bc});
-                    out.cols.push_back(m);
-                    continue;
-                }
-                DevCol d = make_col(rt_, meta.type, (int64_t)cap, nullable, meta.name);
-                if (d.valid) zero(rt_, const_cast<uint8_t *>(d.valid), d.hold_valid->bytes());
-                od.c[od.n++] = OutColDev{s.data, meta.nullable ? s.valid : nullptr, 0, const_cast<void *>(d.data),
-                                         (uint32_t *)d.valid, meta.type.width(), 1};
-                out.cols.push_back(d);
+                column(s, meta.type, meta.name, meta.nullable ? s.valid : nullptr, 1, bc, meta.nullable || build_nullable);
             }
-        }
-        DBuf idx[2];
         for (const VarOut &v : vars)
-            if (!idx[v.side].get()) {
-                idx[v.side] = DBuf(rt_, (size_t)cap * 8);
-                od.c[od.n++] = OutColDev{nullptr, nullptr, 0, idx[v.side].get(), nullptr, 8, 3 + v.side};
-            }
-        zero(rt_, cnt.get(), 8);
-        clear_status(rt_);
-        if (n > 0) {
-            auto *count = cnt.as<unsigned long long>();
-            if (pairs) {
-                if (build_rows_ > 0 || jt == KRV_JOIN_LEFT_OUTER || jt == KRV_JOIN_FULL_OUTER) {
-                    // An empty build still has an all-empty table: every lookup misses.
-                    auto *mc = counters_dev_.as<unsigned long long>() + 6;
-                    uint8_t *marks = marks_.get() ? marks_.as<uint8_t>() : nullptr;
-                    const int pad = jt == KRV_JOIN_LEFT_OUTER || jt == KRV_JOIN_FULL_OUTER;
-                    // unique build keys: at most one output row per probe row
-                    const bool unique = build_rows_ > 0 && counters_.build_keys == indexed_rows_;
-                    if (fast && unique && !marks && pk.null_safe == 0 && !filt &&
-                        (jt == KRV_JOIN_INNER || jt == KRV_JOIN_LEFT_OUTER)) {
-                        const int fgrid = grid_for(rt_, ceil_div(n, kFastRows), kFastThreads, 8);
-                        const DirectDev dd{direct_.as<uint32_t>(), key_lo_, direct_span_};
-                        if (dd.row)
-                            probe_fast_kernel<true><<<fgrid, kFastThreads, 0, rt_->stream>>>(
-                                pk, bk, n, slots, mask_, spec_.seed, dd, od, cap, count, pad);
-                        else
-                            probe_fast_kernel<false><<<fgrid, kFastThreads, 0, rt_->stream>>>(
-                                pk, bk, n, slots, mask_, spec_.seed, dd, od, cap, count, pad);
-                    } else {
-                        launch_pairs(fast, filt, grid, threads, pk, bk, n, od, cap, count, marks, pad,
-                                     spec_.single_match, mc, fd);
-                    }
-                    rt_->launches++;
-                    check_launch("probe_pairs_kernel");
-                }
-            } else {
-                const int kind = jt == KRV_JOIN_LEFT_SEMI ? 0 : jt == KRV_JOIN_LEFT_ANTI ? 1 : 2;
-                const unsigned long long *sl = slots;
-                const uint64_t mask = mask_;
-                const uint32_t *nx = next_.as<uint32_t>();
-                const int empty = build_rows_ == 0, hn = any_null_build_;
-                if (fast && filt)
-                    probe_rows_kernel<true, true><<<grid, threads, 0, rt_->stream>>>(
-                        pk, bk, n, sl, mask, spec_.seed, od, cap, count, kind, empty, hn, nx, fd);
-                else if (fast)
-                    probe_rows_kernel<true, false><<<grid, threads, 0, rt_->stream>>>(
-                        pk, bk, n, sl, mask, spec_.seed, od, cap, count, kind, empty, hn, nx, fd);
-                else if (filt)
-                    probe_rows_kernel<false, true><<<grid, threads, 0, rt_->stream>>>(
-                        pk, bk, n, sl, mask, spec_.seed, od, cap, count, kind, empty, hn, nx, fd);
-                else
-                    probe_rows_kernel<false, false><<<grid, threads, 0, rt_->stream>>>(
-                        pk, bk, n, sl, mask, spec_.seed, od, cap, count, kind, empty, hn, nx, fd);
-                rt_->launches++;
-                check_launch("probe_rows_kernel");
-            }
+            if (!idx[v.side].get()) idx[v.side] = DBuf(rt_, (size_t)std::max<int64_t>(m, 1) * 8);
+        for (int side = 0; side < 2; side++)
+            if (idx[side].get()) od.c[od.n++] = OutColDev{nullptr, nullptr, 0, idx[side].get(), nullptr, 8, 3 + side};
+        if (m == 0 || none) return;
+        for (int64_t row0 = 0; row0 < n; row0 += chunk) {
+            const int64_t rows = std::min(chunk, n - row0);
+            if (chunk < n)
+                launch_lookup(how, row0, rows, head.as<uint32_t>(), how == kChains ? cnt.as<uint32_t>() : nullptr, nullptr,
+                              nullptr, pads && pairs, kind, nullptr);
+            E.row0 = row0;
+            E.rows = rows;
+            E.head = head.as<uint32_t>();
+            E.cnt = cnt.as<uint32_t>();
+            E.tiles = tiles.as<unsigned long long>() + row0 / kTileRows;
+            E.next = next_.as<uint32_t>();
+            E.pad = pads && pairs;
+            launch_emit(how, E, od);
         }
-        const unsigned long long got = read_scalar<unsigned long long>(rt_, cnt.get());
-        const uint32_t st = take_status(rt_);
-        if (st & ST_TOO_MANY) fail(KRV_TOO_MANY_ROWS, "SCALAR_SUBQUERY_TOO_MANY_ROWS: a probe row matched more than one build row");
-        if (got <= cap) {
-            out.rows = (int64_t)got;
-            for (DevCol &c : out.cols) c.length = out.rows;
-            for (const VarOut &v : vars) {
-                const DevCol m = out.cols[v.pos];
-                out.cols[v.pos] = var_gather(rt_, var_src(v.side, v.col, &in), idx[v.side].as<long long>(), out.rows,
-                                             m.type, m.nullable, m.name);
-            }
-            counters_.output_rows += out.rows;
-            remember_shape(out);
-            return out;
+    };
+    // Where a probe row has at most one output row, columns of n rows hold
+    // the output and one wait, after everything is queued, tells its size.
+    // Duplicate build keys wait for the size first.
+    int64_t m = -1;
+    if (how != kChains) {
+        try {
+            emit(n);
+        } catch (const Error &e) {
+            if (e.code != KRV_NEED_MEMORY) throw;
+            idx[0] = DBuf();
+            idx[1] = DBuf();
+            m = total();  // the rows there are may still fit
         }
-        cap = got;  // output larger than guessed: run again with room for all of it
+    } else {
+        m = total();
     }
-    fail(KRV_INTERNAL, "join output did not converge");
+    if (m < 0) m = total();
+    else emit(m);
+    out.rows = m;
+    for (DevCol &c : out.cols) c.length = m;
+    for (const VarOut &v : vars) {
+        const DevCol meta = out.cols[v.pos];
+        out.cols[v.pos] = var_gather(rt_, var_src(v.side, v.col, &in), idx[v.side].as<long long>(), m, meta.type,
+                                     meta.nullable, meta.name);
+    }
+    counters_.output_rows += m;
+    remember_shape(out);
+    emitting_ = how == kChains && m > 0;
+    return out;
 }
 
 DevBatch HashJoin::finish() {

@@ -43,6 +43,17 @@ __host__ __device__ __forceinline__ uint64_t normalize_f64_bits(uint64_t bits) {
     return bits;
 }
 
+// ---- join table slots -------------------------------------------------------------
+// A slot is 0 (empty) or: bit 63, the key has more than one build row (its
+// chain goes on in `next`: a probe of a key without the bit reads no link);
+// bits 32..62, the top bits of g as a tag; bits 0..31, the newest build row + 1.
+constexpr unsigned long long kSlotChained = 1ull << 63;
+__host__ __device__ __forceinline__ uint32_t slot_tag(uint64_t g) { return (uint32_t)(g >> 32) & 0x7FFFFFFFu; }
+__host__ __device__ __forceinline__ bool slot_matches(unsigned long long s, uint32_t tag) {
+    return ((uint32_t)(s >> 32) & 0x7FFFFFFFu) == tag;
+}
+__host__ __device__ __forceinline__ uint32_t slot_row(unsigned long long s) { return (uint32_t)s - 1u; }
+
 // ---- XXH64 (seed 0) of fixed-width little-endian values --------------------
 // The public XXH64 algorithm's short-input path for 8 bytes, as the engine's
 // runtime filters hash int64 keys (crates/krishiv-kernels/src/hash/

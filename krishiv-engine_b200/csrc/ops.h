@@ -141,6 +141,8 @@ class HashJoin {
     const krv_join_spec &spec() const { return spec_; }
     bool built() const { return built_; }
     bool has_residual() const { return residual_set_; }
+    // Work queued by the last probe still reads its input batch.
+    bool emitting() const { return emitting_; }
     // Takes the probe key columns and the output projection of `s` (a plan
     // that probes one built table with batches of another shape).
     void set_probe_shape(const krv_join_spec &s) {
@@ -234,7 +236,7 @@ class HashJoin {
     int64_t arena_cap_ = 0;
     DevBatch arena_;                    // view of the arena
     bool have_schema_ = false;
-    DBuf slots_, next_, marks_, counters_dev_;
+    DBuf slots_, next_, marks_;
     DBuf direct_;  // unique dense keys: key - key_lo_ -> build row
     unsigned long long direct_span_ = 0;
     uint64_t mask_ = 0;
@@ -242,6 +244,7 @@ class HashJoin {
     bool built_ = false;
     bool any_null_build_ = false;
     bool finished_ = false;
+    bool emitting_ = false;
     std::vector<DType> probe_types_;
     std::vector<std::string> probe_names_;
     std::vector<bool> probe_nullable_;

@@ -117,13 +117,13 @@ struct TickDev {
 
 __device__ __forceinline__ uint32_t table_head(const TableView &t, long long k) {
     const uint64_t g = finalize(hash_word((uint64_t)k), t.seed);
-    const unsigned long long tag = g >> 32;
+    const uint32_t tag = slot_tag(g);
     uint64_t pos = g & t.mask;
     for (uint64_t p = 0; p <= t.mask; p++) {
         const unsigned long long s = __ldg(t.slots + pos);
         if (s == 0) return kNoRow;
-        if ((s >> 32) == tag) {
-            const uint32_t o = (uint32_t)(s & 0xFFFFFFFFull) - 1u;
+        if (slot_matches(s, tag)) {
+            const uint32_t o = slot_row(s);
             if (__ldg(t.keys + o) == k) return o;
         }
         pos = (pos + 1) & t.mask;
@@ -156,7 +156,7 @@ __global__ void records_kernel(const unsigned long long *slots, uint64_t n, cons
         const unsigned long long s = slots[i];
         Record r{0, -1, 0};
         if (s) {
-            const uint32_t row = (uint32_t)(s & 0xFFFFFFFFull) - 1u;
+            const uint32_t row = slot_row(s);
             r.key = keys[row];
             r.gid = gid[row];
         }
