@@ -102,34 +102,37 @@ __device__ uint64_t dict_hash(const DictDev &D, int64_t i) {
     return fold(h, kFinish);
 }
 
-// Row i's key equals code `code`'s stored key. The stored keys are read
-// through L2 (ld.global.cg): they were written by another thread after this
-// SM may have cached their neighbours.
-__device__ bool dict_eq(const DictDev &D, int64_t i, uint64_t code) {
+// A stored key's value: through L2 (ld.global.cg) while keys are inserted,
+// since another thread may have written it after this SM cached its
+// neighbours; through L1 in a kernel that only looks keys up.
+template <bool CACHED, class T> __device__ __forceinline__ T stored(const T *p) { return CACHED ? *p : __ldcg(p); }
+
+// Row i's key equals code `code`'s stored key.
+template <bool CACHED> __device__ bool dict_eq(const DictDev &D, int64_t i, uint64_t code) {
     for (int c = 0; c < D.n; c++) {
         const DictKeyIn &K = D.in[c];
         const DictStore &S = D.st[c];
         const bool v = bit_get(K.valid, K.voff, i);
-        if (v != (__ldcg(S.valid + code) != 0)) return false;
+        if (v != (stored<CACHED>(S.valid + code) != 0)) return false;
         if (!v) continue;
         if (K.width == 0) {
             const int32_t *offs = static_cast<const int32_t *>(K.data);
             const int32_t o = offs[i], len = offs[i + 1] - o;
-            if (len != __ldcg(S.str_len + code)) return false;
+            if (len != stored<CACHED>(S.str_len + code)) return false;
             const uint8_t *a = K.bytes + o;
-            const uint8_t *b = D.heap + __ldcg(S.str_off + code);
+            const uint8_t *b = D.heap + stored<CACHED>(S.str_off + code);
             for (int32_t k = 0; k < len; k++)
-                if (a[k] != __ldcg(b + k)) return false;
+                if (a[k] != stored<CACHED>(b + k)) return false;
         } else {
             uint64_t w0, w1, s0, s1 = 0;
             fixed_words(K, i, w0, w1);
             if (K.width == 4) {
-                s0 = __ldcg(static_cast<const uint32_t *>(S.vals) + code);
+                s0 = stored<CACHED>(static_cast<const uint32_t *>(S.vals) + code);
             } else if (K.width == 8) {
-                s0 = __ldcg(static_cast<const unsigned long long *>(S.vals) + code);
+                s0 = stored<CACHED>(static_cast<const unsigned long long *>(S.vals) + code);
             } else {
-                s0 = __ldcg(static_cast<const unsigned long long *>(S.vals) + 2 * code);
-                s1 = __ldcg(static_cast<const unsigned long long *>(S.vals) + 2 * code + 1);
+                s0 = stored<CACHED>(static_cast<const unsigned long long *>(S.vals) + 2 * code);
+                s1 = stored<CACHED>(static_cast<const unsigned long long *>(S.vals) + 2 * code + 1);
             }
             if (w0 != s0 || w1 != s1) return false;
         }
@@ -178,9 +181,13 @@ __device__ void dict_store(const DictDev &D, int64_t i, uint64_t code) {
 
 // The code of every row's key: found, or (insert) claimed in the table and
 // given the next dense code; -1 for a key not in the table (lookup only) or
-// past the capacities the host sized (status bits say which).
-__global__ void __launch_bounds__(256) dict_encode_kernel(DictDev D, int64_t n, int insert, long long *codes) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+// past the capacities the host sized (status bits say which). The rows are
+// those listed in rows_idx, else every `step`-th; codes (none when null) are
+// stored by row.
+__global__ void __launch_bounds__(256) dict_encode_kernel(DictDev D, int64_t n, int insert, long long *codes, int64_t step,
+                                                          const uint32_t *rows_idx) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = rows_idx ? (int64_t)rows_idx[j] : j * step;
         const uint64_t h = dict_hash(D, i);
         const unsigned long long tag = h >> 32;
         uint64_t pos = h & D.mask;
@@ -221,14 +228,155 @@ __global__ void __launch_bounds__(256) dict_encode_kernel(DictDev D, int64_t n, 
                     }
                     __threadfence();
                 }
-                if (lo != kDictDead && dict_eq(D, i, lo - 1)) {
+                if (lo != kDictDead && dict_eq<false>(D, i, lo - 1)) {
                     code = (long long)(lo - 1);
                     break;
                 }
             }
             pos = (pos + 1) & D.mask;
         }
-        codes[i] = code;
+        if (codes) codes[i] = code;
+    }
+}
+
+// The codes of keys that a sample of the batch has already put into the
+// table, which nothing writes meanwhile: slots and stored keys come from L1
+// (a few keys' worth), where the inserting kernel reads them from L2 every
+// time. Rows of keys the table does not hold are listed for that kernel.
+// Measured on B200, 6M rows of two int32 columns, 6 keys: 0.064 ms, the
+// inserting kernel 0.12 ms (0.075 ms with each row hashed and compared alone,
+// its loads one after the other).
+constexpr int kLookRows = 4;  // rows per thread: their loads are in flight together
+constexpr int kLookThreads = 256;
+template <bool FIXED>
+__global__ void __launch_bounds__(kLookThreads) dict_lookup_kernel(DictDev D, int64_t n, long long *codes, uint32_t *miss_rows,
+                                                                   unsigned long long *misses) {
+    constexpr int U = kLookRows;
+    const int64_t stride = (int64_t)gridDim.x * kLookThreads * U;
+    for (int64_t b0 = blockIdx.x * (int64_t)kLookThreads * U; b0 < n; b0 += stride) {
+        const int64_t i0 = b0 + threadIdx.x;
+        uint64_t h[U];
+        long long code[U];
+        if (FIXED) {  // column by column: a column's width and bitmap are looked at once for all rows
+#pragma unroll
+            for (int u = 0; u < U; u++) h[u] = 0;
+            for (int c = 0; c < D.n; c++) {
+                const DictKeyIn &K = D.in[c];
+                uint64_t w0[U], w1[U];
+                uint32_t null = 0;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int64_t i = i0 + u * kLookThreads;
+                    w0[u] = w1[u] = 0;
+                    if (i < n) fixed_words(K, i, w0[u], w1[u]);
+                }
+                if (K.valid) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int64_t i = i0 + u * kLookThreads;
+                        if (i < n && !bit_get(K.valid, K.voff, i)) null |= 1u << u;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    h[u] = mix(h[u], (null >> u) & 1u ? kNullHash : w0[u]);
+                    if (K.width == 16 && !((null >> u) & 1u)) h[u] = mix(h[u], w1[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) h[u] = fold(h[u], kFinish);
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) h[u] = i0 + u * kLookThreads < n ? dict_hash(D, i0 + u * kLookThreads) : 0;
+        }
+        // The first slot of each row that bears its tag, then its key compared,
+        // again column by column; what that does not settle is walked on alone.
+        uint32_t walk = 0;
+        uint64_t pos[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t i = i0 + u * kLookThreads;
+            pos[u] = h[u] & D.mask;
+            code[u] = -1;
+            if (i >= n) continue;
+            const unsigned long long s = D.slots[pos[u]];
+            const uint32_t lo = (uint32_t)s;
+            if (s == 0) continue;  // no such key
+            if (FIXED && (uint32_t)(s >> 32) == (uint32_t)(h[u] >> 32) && lo != kDictDead && lo != kDictPending) code[u] = (long long)(lo - 1);
+            else walk |= 1u << u;
+        }
+        if (FIXED) {
+            uint32_t differs = 0;
+            for (int c = 0; c < D.n; c++) {
+                const DictKeyIn &K = D.in[c];
+                const DictStore &S = D.st[c];
+                uint64_t w0[U], w1[U], s0[U], s1[U];
+                uint32_t null = 0;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    w0[u] = w1[u] = s0[u] = s1[u] = 0;
+                    if (code[u] >= 0) fixed_words(K, i0 + u * kLookThreads, w0[u], w1[u]);
+                }
+                if (K.width == 4) {
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (code[u] >= 0) s0[u] = static_cast<const uint32_t *>(S.vals)[code[u]];
+                } else if (K.width == 8) {
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (code[u] >= 0) s0[u] = static_cast<const unsigned long long *>(S.vals)[code[u]];
+                } else {
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (code[u] >= 0) {
+                            s0[u] = static_cast<const unsigned long long *>(S.vals)[2 * code[u]];
+                            s1[u] = static_cast<const unsigned long long *>(S.vals)[2 * code[u] + 1];
+                        }
+                }
+                if (K.valid) {
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (code[u] >= 0 && !bit_get(K.valid, K.voff, i0 + u * kLookThreads)) null |= 1u << u;
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (code[u] < 0) continue;
+                    const uint32_t is_null = (null >> u) & 1u, was_null = S.valid[code[u]] == 0 ? 1u : 0u;
+                    if (is_null != was_null || (!is_null && (w0[u] != s0[u] || w1[u] != s1[u]))) differs |= 1u << u;
+                }
+            }
+            walk |= differs;
+        }
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t i = i0 + u * kLookThreads;
+            if (i >= n) continue;
+            if ((walk >> u) & 1u) {
+                const uint32_t tag = (uint32_t)(h[u] >> 32);
+                code[u] = -1;
+                for (uint64_t probes = 0; probes <= D.mask; probes++) {
+                    const unsigned long long s = D.slots[pos[u]];
+                    if (s == 0) break;
+                    const uint32_t lo = (uint32_t)s;
+                    if ((uint32_t)(s >> 32) == tag && lo != kDictDead && lo != kDictPending && dict_eq<true>(D, i, lo - 1)) {
+                        code[u] = (long long)(lo - 1);
+                        break;
+                    }
+                    pos[u] = (pos[u] + 1) & D.mask;
+                }
+            }
+            codes[i] = code[u];
+            any = any || code[u] < 0;
+        }
+        if (!__any_sync(0xFFFFFFFFu, any)) continue;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t i = i0 + u * kLookThreads;
+            const bool miss = i < n && code[u] < 0;
+            const unsigned long long at = warp_alloc(misses, miss, 0xFFFFFFFFu);
+            if (miss) miss_rows[at] = (uint32_t)i;
+        }
     }
 }
 
@@ -293,10 +441,8 @@ class KeyDict {
                 fail(KRV_UNSUPPORTED, "group key of type " + m.type.format());
         }
         store_.resize(meta_.size());
-        ncodes_ = DBuf(rt_, 8);
-        heap_used_ = DBuf(rt_, 8);
-        KRV_CUDA(cudaMemsetAsync(ncodes_.get(), 0, 8, rt_->stream));
-        KRV_CUDA(cudaMemsetAsync(heap_used_.get(), 0, 8, rt_->stream));
+        ctr_ = DBuf(rt_, 32);
+        KRV_CUDA(cudaMemsetAsync(ctr_.get(), 0, 32, rt_->stream));
     }
 
     int64_t size() const { return count_; }
@@ -321,12 +467,8 @@ class KeyDict {
                 KRV_CUDA(cudaMemsetAsync(codes.get(), 0xFF, (size_t)n * 8, rt_->stream));
                 return codes;
             }
-            DictDev D = dev(b, cols);
-            clear_status(rt_);
-            dict_encode_kernel<<<grid_for(rt_, n, 256, 8), 256, 0, rt_->stream>>>(D, n, 0, codes.as<long long>());
-            rt_->launches++;
-            check_launch("dict_encode_kernel");
-            if (take_status(rt_) & ST_TIMEOUT) fail(KRV_TIMEOUT, "group keys: a wait for a code gave up");
+            run_encode(dev(b, cols), n, 0, codes.as<long long>(), 1, nullptr);
+            read_counters();
             return codes;
         }
         int64_t heap_need = 0;
@@ -342,20 +484,36 @@ class KeyDict {
                 heap_need += std::max<int32_t>(0, ends[1] - ends[0]);
             }
         }
+        // A large batch usually repeats its keys: a strided sample of the rows
+        // is inserted first. When it holds few keys, the rows are looked up and
+        // only those of other keys inserted, with room for that many; else the
+        // table gets room for every row being new.
+        const int64_t m = kSampleRows;
+        if (n >= 4 * m && n < (int64_t)0xFFFFFFFFll) {
+            const int64_t before = count_;
+            reserve(count_ + m, heap_used_host_ + heap_need);
+            run_encode(dev(b, cols), m, 1, nullptr, n / m, nullptr);
+            read_counters();
+            if (count_ - before <= m / 8) {
+                DBuf miss_rows(rt_, (size_t)n * 4);
+                KRV_CUDA(cudaMemsetAsync(ctr_.as<unsigned long long>() + 2, 0, 8, rt_->stream));
+                const bool fixed = std::none_of(meta_.begin(), meta_.end(), [](const DevCol &k) { return k.type.var(); });
+                const auto kernel = fixed ? dict_lookup_kernel<true> : dict_lookup_kernel<false>;
+                kernel<<<grid_for(rt_, ceil_div(n, kLookRows), kLookThreads, 8), kLookThreads, 0, rt_->stream>>>(
+                    dev(b, cols), n, codes.as<long long>(), miss_rows.as<uint32_t>(), ctr_.as<unsigned long long>() + 2);
+                rt_->launches++;
+                check_launch("dict_lookup_kernel");
+                const int64_t misses = read_counters();
+                if (misses == 0) return codes;
+                reserve(count_ + misses, heap_used_host_ + heap_need);
+                run_encode(dev(b, cols), misses, 1, codes.as<long long>(), 1, miss_rows.as<uint32_t>());
+                read_counters();
+                return codes;
+            }
+        }
         reserve(count_ + n, heap_used_host_ + heap_need);
-        DictDev D = dev(b, cols);
-        clear_status(rt_);
-        dict_encode_kernel<<<grid_for(rt_, n, 256, 8), 256, 0, rt_->stream>>>(D, n, 1, codes.as<long long>());
-        rt_->launches++;
-        check_launch("dict_encode_kernel");
-        unsigned long long got[2];
-        read_device(rt_, ncodes_.get(), 8, &got[0]);
-        read_device(rt_, heap_used_.get(), 8, &got[1]);
-        const uint32_t st = take_status(rt_);
-        if (st & ST_TIMEOUT) fail(KRV_TIMEOUT, "group keys: a wait for a code gave up");
-        if (st & ST_CAPACITY) fail(KRV_INTERNAL, "group keys: capacity exceeded");
-        count_ = (int64_t)got[0];
-        heap_used_host_ = (int64_t)got[1];
+        run_encode(dev(b, cols), n, 1, codes.as<long long>(), 1, nullptr);
+        read_counters();
         return codes;
     }
 
@@ -430,9 +588,28 @@ class KeyDict {
     }
 
   private:
+    static constexpr int64_t kSampleRows = 16384;
     struct Store {
         DBuf vals, valid, str_off, str_len;
     };
+
+    void run_encode(const DictDev &D, int64_t n, int insert, long long *codes, int64_t step, const uint32_t *rows_idx) {
+        dict_encode_kernel<<<grid_for(rt_, n, 256, 8), 256, 0, rt_->stream>>>(D, n, insert, codes, step, rows_idx);
+        rt_->launches++;
+        check_launch("dict_encode_kernel");
+    }
+    // Codes and heap bytes in use, and what the kernels reported (one wait);
+    // the last lookup's missing rows are returned.
+    int64_t read_counters() {
+        unsigned long long c[4];
+        read_device(rt_, ctr_.get(), sizeof(c), c);
+        const uint32_t st = (uint32_t)c[3];
+        if (st & ST_TIMEOUT) fail(KRV_TIMEOUT, "group keys: a wait for a code gave up");
+        if (st & ST_CAPACITY) fail(KRV_INTERNAL, "group keys: capacity exceeded");
+        count_ = (int64_t)c[0];
+        heap_used_host_ = (int64_t)c[1];
+        return (int64_t)c[2];
+    }
 
     DictDev dev(const DevBatch &b, const std::vector<int> &cols) {
         DictDev D{};
@@ -452,12 +629,12 @@ class KeyDict {
         D.slots = slots_.as<unsigned long long>();
         D.mask = slot_count_ - 1;
         D.hashes = hashes_.as<unsigned long long>();
-        D.ncodes = ncodes_.as<unsigned long long>();
+        D.ncodes = ctr_.as<unsigned long long>();
         D.code_cap = (unsigned long long)code_cap_;
         D.heap = heap_.as<uint8_t>();
-        D.heap_used = heap_used_.as<unsigned long long>();
+        D.heap_used = ctr_.as<unsigned long long>() + 1;
         D.heap_cap = (unsigned long long)heap_cap_;
-        D.status = status_word(rt_);
+        D.status = reinterpret_cast<uint32_t *>(ctr_.as<unsigned long long>() + 3);
         return D;
     }
 
@@ -526,7 +703,8 @@ class KeyDict {
     Runtime *rt_;
     std::vector<DevCol> meta_;
     std::vector<Store> store_;
-    DBuf slots_, hashes_, ncodes_, heap_, heap_used_;
+    DBuf slots_, hashes_, heap_;
+    DBuf ctr_;  // codes, heap bytes, missing rows of a lookup, status bits (a set bit fails the dictionary)
     uint64_t slot_count_ = 0;
     int64_t code_cap_ = 0, heap_cap_ = 0;
     int64_t count_ = 0, heap_used_host_ = 0;
