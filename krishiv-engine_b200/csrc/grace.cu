@@ -43,7 +43,7 @@ constexpr int kMaxLevel = 6;
 
 struct PartCol {
     const void *src;
-    void *dst;
+    void *dst;  // compact_unmatched_kernel's; the scatter's are in `to`
     int width;  // 4 or 8
 };
 struct PartArgs {
@@ -62,6 +62,7 @@ struct PartArgs {
     uint8_t *bucket;    // with kFilterTest: each row's bucket, written by the histogram pass for the scatter
     PartCol c[kMaxCols];
     int ncols;
+    void *const *to;    // the scatter's destinations: column c of bucket p goes to to[c * (nparts + 2) + p]
 };
 constexpr int kFilterNone = 0, kFilterInsert = 1, kFilterTest = 2;
 
@@ -96,6 +97,12 @@ __global__ void __launch_bounds__(256) part_hist_kernel(PartArgs A, unsigned lon
 // Tiles of kPartTile rows: rank every row within its partition in shared
 // memory, claim each partition's run of the output with one atomic per tile,
 // then write the tile column by column in partition order (coalesced runs).
+// Every bucket has a destination of its own, so a partition's rows go where
+// they are needed next: a resident build partition's into its table's arena,
+// the rows that spill side by side into one buffer that leaves with one copy
+// per column. Measured on B200, 50M build rows of 24 bytes, 3 of 8 partitions
+// spilling: 7 ms, at the host link's rate, where a copy per partition and
+// column took 26 ms; a probe slice of 1.56M rows takes 40 us.
 //
 // With kFilterInsert every non-NULL key also goes into the Bloom filter (one
 // 32-byte block per key: 8 lanes of a warp set one word each), so that the
@@ -166,11 +173,60 @@ __global__ void __launch_bounds__(kPartThreads) part_scatter_kernel(PartArgs A, 
             for (unsigned j = threadIdx.x; j < total; j += kPartThreads) {
                 const int p = s_part[j];
                 const unsigned long long at = s_base[p] + (j - s_off[p]);
-                if (C.width == 8) static_cast<unsigned long long *>(C.dst)[at] = s_val[j];
-                else static_cast<uint32_t *>(C.dst)[at] = (uint32_t)s_val[j];
+                void *dst = A.to[c * (A.nparts + 2) + p];
+                if (C.width == 8) static_cast<unsigned long long *>(dst)[at] = s_val[j];
+                else static_cast<uint32_t *>(dst)[at] = (uint32_t)s_val[j];
             }
             __syncthreads();
         }
+    }
+}
+
+// ---- rows coming back from host memory ---------------------------------------------
+// A group of spilled chunks read in place from page-locked memory, all chunks
+// and columns in one launch. Bound by the host link, which 16 blocks with 8
+// loads to a thread in flight keep busy (1.9 GB of 200 KB pieces on B200: 40
+// GB/s, 16, 48 and 148 blocks alike, where one copy per piece reached 22), so
+// most SMs are left to the join of the group before.
+constexpr int kGatherThreads = 256;
+constexpr int kGatherBlocks = 16;
+constexpr int kGatherWords = 8;  // words per thread and tile, in flight together
+struct GatherRun {
+    const void *src;
+    void *dst;
+    int64_t words;
+    int32_t width, pad;
+    int64_t tile0;  // its first tile of kGatherThreads x kGatherWords words
+};
+
+template <class T> __device__ __forceinline__ void gather_tile(const GatherRun &R, int64_t w0) {
+    const T *src = static_cast<const T *>(R.src);
+    T *dst = static_cast<T *>(R.dst);
+    T v[kGatherWords];
+#pragma unroll
+    for (int u = 0; u < kGatherWords; u++) {
+        const int64_t i = w0 + u * kGatherThreads + threadIdx.x;
+        v[u] = i < R.words ? __ldcs(src + i) : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < kGatherWords; u++) {
+        const int64_t i = w0 + u * kGatherThreads + threadIdx.x;
+        if (i < R.words) dst[i] = v[u];
+    }
+}
+
+__global__ void __launch_bounds__(kGatherThreads) gather_kernel(const GatherRun *runs, int n, int64_t tiles) {
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        int lo = 0, hi = n - 1;  // the last run whose first tile is at most t
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (runs[mid].tile0 <= t) lo = mid;
+            else hi = mid - 1;
+        }
+        const GatherRun R = runs[lo];
+        const int64_t w0 = (t - R.tile0) * (kGatherThreads * kGatherWords);
+        if (R.width == 8) gather_tile<unsigned long long>(R, w0);
+        else gather_tile<uint32_t>(R, w0);
     }
 }
 
@@ -381,10 +437,21 @@ int radix_for(int64_t build_rows, int64_t row_bytes, int64_t budget) {
 
 // ---- the operator ------------------------------------------------------------------
 class GraceJoin {
-    // One partition's rows of a partitioned slice (views of its buffers).
-    struct Segment {
-        DevBatch batch;
+    // A batch whose buckets have been counted: what the scatter needs.
+    struct Counted {
+        PartArgs args{};
+        DBuf ctr, bucket;
+        std::vector<unsigned long long> rows;  // per bucket: partitions, NULL keys, ruled-out rows
+        DBuf to;                               // the scatter's destinations
+    };
+    // Rows of some buckets side by side: owned columns of their own.
+    struct Rows {
+        std::vector<std::shared_ptr<DBuf>> cols;
+        std::vector<std::pair<int, int64_t>> runs;  // bucket, rows
         int64_t rows = 0;
+        void add(int bucket, int64_t n) {
+            if (n) runs.push_back({bucket, n}), rows += n;
+        }
     };
 
   public:
@@ -411,6 +478,8 @@ class GraceJoin {
         for (auto &f : inflight_) cudaEventDestroy(f.done);
         inflight_.clear();
         if (prefetch_.ready) cudaEventDestroy(prefetch_.ready);
+        if (later_.ready) cudaEventDestroy(later_.ready);
+        if (next_build_.ready) cudaEventDestroy(next_build_.ready);
         cudaStreamDestroy(cs_);
         for (auto &b : host_blocks_) rt_->host_pool->give(b.first, b.second);
     }
@@ -425,18 +494,31 @@ class GraceJoin {
     }
 
     void build_slice(const DevBatch &b) {
-        std::vector<Segment> segs = partition(b, spec_.build_keys[0], 0, parts_bits_, false, bloom_ ? kFilterInsert : kFilterNone);
+        Counted k = count(b, spec_.build_keys[0], 0, parts_bits_, false, bloom_ ? kFilterInsert : kFilterNone);
+        std::vector<void *> to(k.args.ncols * k.rows.size(), nullptr);
+        Rows host;
         for (int p = 0; p < nparts_; p++) {
-            Segment &s = segs[p];
-            if (s.rows == 0) continue;
+            const int64_t n = (int64_t)k.rows[p];
+            if (n == 0) continue;
             Part &P = parts_[p];
             if (P.spilled) {
-                P.build_host.push_back(spill(s));
-            } else {
-                P.join->build_push(s.batch);
-                P.build_rows += s.rows;
+                host.add(p, n);
+            } else {  // straight into the partition's table
+                void *dst[kMaxCols];
+                P.join->build_reserve(n, dst);
+                for (int c = 0; c < k.args.ncols; c++) to[c * k.rows.size() + p] = dst[c];
             }
         }
+        place(host, build_types_, k, to);
+        scatter(k, to);
+        for (int p = 0; p < nparts_; p++) {
+            Part &P = parts_[p];
+            if (P.spilled || k.rows[p] == 0) continue;
+            P.join->build_commit((int64_t)k.rows[p]);
+            P.build_rows += (int64_t)k.rows[p];
+        }
+        std::vector<HostChunk> chunks = spill(host, build_types_);
+        for (size_t i = 0; i < chunks.size(); i++) parts_[host.runs[i].first].build_host.push_back(chunks[i]);
         enforce_residency();
     }
 
@@ -470,58 +552,120 @@ class GraceJoin {
         check_shape(in, probe_types_, spec_.probe_keys[0], "probe");
         counters_.probe_rows += in.rows;
         std::vector<DevBatch> out;
-        int64_t out_rows = 0;
+        Share share;
+        share.rows_left = in.rows;
         // The batches go out as they are, one per call of krv_join_probe: one
         // batch would cost a copy of them all (and its allocation).
-        for (int64_t from = 0; from < in.rows; from += slice_rows()) probe_slice(slice(in, from), out, out_rows);
+        for (int64_t from = 0; from < in.rows; from += slice_rows()) probe_slice(slice(in, from), out, share);
+        KRV_CUDA(cudaStreamSynchronize(rt_->stream));  // the caller's columns are its own again
         return out;
     }
 
-    // One slice: NULL-key rows padded now (left outer); rows of resident
-    // partitions joined now while this call's output stays under a quarter
-    // of the budget, else deferred to host memory like those of spilled
-    // partitions (and joined at finish by the same resident tables).
-    void probe_slice(const DevBatch &in, std::vector<DevBatch> &out, int64_t &out_rows) {
-        std::vector<Segment> segs = partition(in, spec_.probe_keys[0], 0, parts_bits_, true, bloom_ ? kFilterTest : kFilterNone);
-        Segment &nulls = segs[nparts_];
-        if (nulls.rows > 0 && spec_.join_type == KRV_JOIN_LEFT_OUTER) {
-            out_rows += nulls.rows;
-            keep(out, null_join_->probe(with_null_keys(nulls)));
+    // What a probe call has put out so far.
+    struct Share {
+        int64_t bytes = 0;      // of its output batches
+        int64_t rows_left = 0;  // input rows yet to come
+        int64_t rows = 0, ruled_out = 0;
+    };
+
+    // One slice: rows without a match by their NULL key or by the filter
+    // padded now (left outer), rows of resident partitions joined now, while
+    // this call's output stays under an eighth of the budget; what is past
+    // that goes to host memory like the rows of spilled partitions (and is
+    // joined at finish by the same resident tables). Padded rows come first,
+    // those of the slices yet to come too: they are the partition pass's own
+    // copy of the probe columns beside shared NULL columns, so of the same
+    // bytes of output they keep twice as many rows off the host link.
+    void probe_slice(const DevBatch &in, std::vector<DevBatch> &out, Share &share) {
+        const bool left = spec_.join_type == KRV_JOIN_LEFT_OUTER;
+        Counted k = count(in, spec_.probe_keys[0], 0, parts_bits_, left, bloom_ ? kFilterTest : kFilterNone);
+        const int64_t nulls = left ? (int64_t)k.rows[nparts_] : 0;
+        const int64_t ruled_out = left ? (int64_t)k.rows[nparts_ + 1] : 0;
+        counters_filtered_ += (int64_t)k.rows[nparts_ + 1];  // counted whether the rows are kept or dropped
+        const int64_t out_cap = budget_ / 8, pad_bytes = probe_row_bytes();
+        share.rows += in.rows;
+        share.rows_left -= in.rows;
+        share.ruled_out += ruled_out;
+        share.bytes += nulls * pad_bytes;
+        Rows pad, now, host;
+        pad.add(nparts_, nulls);
+        if (share.bytes + ruled_out * pad_bytes <= out_cap) {
+            pad.add(nparts_ + 1, ruled_out);
+            share.bytes += ruled_out * pad_bytes;
+        } else {
+            host.add(nparts_ + 1, ruled_out);
         }
-        // Rows whose key the build side's Bloom filter rules out match no
-        // build row: padded now (left outer), never partitioned or spilled.
-        Segment &ruled_out = segs[nparts_ + 1];
-        counters_filtered_ += last_filtered_;
-        const int64_t out_cap = budget_ / 8 / out_row_bytes();
-        if (ruled_out.rows > 0 && spec_.join_type == KRV_JOIN_LEFT_OUTER) {
-            if (out_rows + ruled_out.rows > out_cap) {
-                pad_later_.push_back(spill(ruled_out));  // past this call's output share: padded at finish
-            } else {
-                out_rows += ruled_out.rows;
-                keep(out, null_join_->probe(ruled_out.batch));
-            }
-        }
+        const double to_come = (double)share.rows_left * (double)share.ruled_out / (double)std::max<int64_t>(share.rows, 1);
+        const double room = (double)out_cap - (double)share.bytes - to_come * (double)pad_bytes;
         const double ratio = out_ratio();
-        std::vector<int> now;  // resident partitions joined by this slice's launch
         double expect = 0;
         for (int p = 0; p < nparts_; p++) {
-            Segment &s = segs[p];
-            if (s.rows == 0) continue;
-            Part &P = parts_[p];
-            if (P.spilled) {
-                P.probe_host.push_back(spill(s));
-            } else if ((double)out_rows + expect >= (double)out_cap) {
-                P.deferred.push_back(spill(s));
+            const int64_t n = (int64_t)k.rows[p];
+            if (!parts_[p].spilled && expect < room) {
+                now.add(p, n);
+                expect += (double)n * ratio * (double)out_row_bytes();
             } else {
-                now.push_back(p);
-                expect += (double)s.rows * ratio;
+                host.add(p, n);
             }
         }
-        if (!now.empty()) {
-            DevBatch o = probe_resident(segs, now, ratio);
-            out_rows += o.rows;
+        std::vector<void *> to(k.args.ncols * k.rows.size(), nullptr);
+        place(pad, probe_types_, k, to);
+        place(now, probe_types_, k, to);
+        place(host, probe_types_, k, to);
+        scatter(k, to);
+        std::vector<HostChunk> chunks = spill(host, probe_types_);
+        for (size_t i = 0; i < chunks.size(); i++) {
+            const int p = host.runs[i].first;
+            if (p > nparts_) pad_later_.push_back(chunks[i]);
+            else if (parts_[p].spilled) parts_[p].probe_host.push_back(chunks[i]);
+            else parts_[p].deferred.push_back(chunks[i]);
+        }
+        if (pad.rows) keep(out, padded(batch_of(pad, probe_types_), nulls));
+        if (now.rows) {
+            DevBatch o = probe_resident(now, ratio);
+            share.bytes += o.rows * out_row_bytes();
             keep(out, std::move(o));
         }
+    }
+
+    // The output rows of probe rows without a match (owned columns), the
+    // first `nulls` of them with a NULL key: their columns as they are, the
+    // build columns NULL (one zeroed buffer that all of them share).
+    DevBatch padded(DevBatch in, int64_t nulls) {
+        DevBatch o;
+        o.rows = in.rows;
+        const int key = spec_.probe_keys[0];
+        const std::vector<int> pcols = projection(spec_.n_probe_out, spec_.probe_out, (int)probe_types_.size());
+        const std::vector<int> bcols = projection(spec_.n_build_out, spec_.build_out, (int)build_types_.size());
+        if (nulls && std::find(pcols.begin(), pcols.end(), key) != pcols.end()) {
+            DevCol &k = in.cols[key];
+            k.hold_valid = std::make_shared<DBuf>(rt_, (size_t)ceil_div(in.rows, 32) * 4 + 8);
+            KRV_CUDA(cudaMemsetAsync(k.hold_valid->get(), 0, k.hold_valid->bytes(), rt_->stream));
+            set_bits(rt_, k.hold_valid->as<uint8_t>(), nulls, in.rows - nulls);
+            k.valid = k.hold_valid->as<uint8_t>();
+            k.valid_off = 0;
+        }
+        for (int pc : pcols) o.cols.push_back(in.cols[pc]);
+        if (!bcols.empty() && (!null_data_ || in.rows > null_rows_)) {
+            null_rows_ = in.rows;
+            null_data_ = std::make_shared<DBuf>(rt_, (size_t)null_rows_ * 8);
+            null_valid_ = std::make_shared<DBuf>(rt_, (size_t)ceil_div(null_rows_, 32) * 4 + 8);
+            KRV_CUDA(cudaMemsetAsync(null_data_->get(), 0, null_data_->bytes(), rt_->stream));
+            KRV_CUDA(cudaMemsetAsync(null_valid_->get(), 0, null_valid_->bytes(), rt_->stream));
+        }
+        for (int bc : bcols) {
+            DevCol c;
+            c.type = build_types_[bc].type;
+            c.name = build_types_[bc].name;
+            c.nullable = true;
+            c.length = in.rows;
+            c.hold_data = null_data_;
+            c.data = null_data_->get();
+            c.hold_valid = null_valid_;
+            c.valid = null_valid_->as<uint8_t>();
+            o.cols.push_back(c);
+        }
+        return o;
     }
 
     // Output rows per probe row of the resident partitions: as observed so
@@ -552,22 +696,20 @@ class GraceJoin {
         return v;
     }
 
-    // The segments `now` of one partitioned slice, each probed against its
-    // resident partition's table, in one launch and one output batch.
-    DevBatch probe_resident(const std::vector<Segment> &segs, const std::vector<int> &now, double ratio) {
+    // A partitioned slice's rows of resident partitions, each probed against
+    // its partition's table, in one launch and one output batch.
+    DevBatch probe_resident(const Rows &now, double ratio) {
         const int key = spec_.probe_keys[0];
         const std::vector<int> pcols = projection(spec_.n_probe_out, spec_.probe_out, (int)probe_types_.size());
         const std::vector<int> bcols = projection(spec_.n_build_out, spec_.build_out, (int)build_types_.size());
         if (pcols.size() + bcols.size() > (size_t)kGMaxOut) fail(KRV_UNSUPPORTED, "more than 16 output columns");
-        const DevBatch &first = segs[now[0]].batch;
         GOutDev od{};
-        for (size_t c = 0; c < first.cols.size(); c++) od.pcol[c] = first.cols[c].hold_data->get();
+        for (size_t c = 0; c < now.cols.size(); c++) od.pcol[c] = now.cols[c]->get();
         od.pkey = static_cast<const long long *>(od.pcol[key]);
         std::vector<GPartDev> hp;
         int64_t tiles = 0, rows = 0;
-        for (int p : now) {
-            const Segment &s = segs[p];
-            const HashJoin &J = *parts_[p].join;
+        for (const auto &run : now.runs) {
+            const HashJoin &J = *parts_[run.first].join;
             const HashJoin::TableDev tv = J.table_dev();
             GPartDev d{};
             d.slots = tv.slots;
@@ -576,11 +718,11 @@ class GraceJoin {
             const DevBatch &arena = J.arena();
             d.bkey = arena.cols.empty() ? nullptr : static_cast<const long long *>(arena.cols[spec_.build_keys[0]].data);
             for (size_t c = 0; c < arena.cols.size() && c < (size_t)kMaxCols; c++) d.bcol[c] = arena.cols[c].data;
-            d.prow0 = (static_cast<const uint8_t *>(s.batch.cols[key].data) - static_cast<const uint8_t *>(od.pcol[key])) / 8;
-            d.rows = s.rows;
+            d.prow0 = rows;
+            d.rows = run.second;
             d.tile0 = tiles;
-            tiles += ceil_div(s.rows, (int64_t)(32 * kGRows));
-            rows += s.rows;
+            tiles += ceil_div(run.second, (int64_t)(32 * kGRows));
+            rows += run.second;
             hp.push_back(d);
         }
         DBuf dparts(rt_, hp.size() * sizeof(GPartDev));
@@ -637,6 +779,12 @@ class GraceJoin {
         return std::max<int64_t>(b, 8);
     }
 
+    int64_t probe_row_bytes() const {
+        int64_t b = 0;
+        for (const DevCol &c : probe_types_) b += c.type.width();
+        return b;
+    }
+
     // Input batches are taken in slices whose partitioned copy and output
     // stay within a sixteenth of the budget (a multiple of 64 rows, so that
     // every slice starts on a byte of the validity bitmaps).
@@ -663,28 +811,23 @@ class GraceJoin {
             for (int p = 0; p < nparts_; p++)
                 if (parts_[p].spilled) tasks_.push_back(Task{0, std::move(parts_[p].build_host), std::move(parts_[p].probe_host)});
         }
-        // Ruled-out rows that did not fit their call's output: padded now.
-        while (pad_chunk_ < pad_later_.size()) {
-            DevBatch o = null_join_->probe(load_group(pad_later_, pad_chunk_));
+        // Ruled-out rows that did not fit their call's output, padded now, then
+        // the deferred rows of resident partitions, by their resident tables.
+        // The next group crosses the host link while this one is joined.
+        while (later_.pending || start_later()) {
+            const int p = later_part_;
+            DevBatch pb = take(later_);
+            start_later();
+            DevBatch o = p < 0 ? padded(std::move(pb), 0) : parts_[p].join->probe(pb);
+            if (later_part_ != p || !later_.pending)
+                for (int q = 0; q < (later_.pending ? later_part_ : nparts_); q++) parts_[q].join.reset();  // done
             counters_.output_rows += o.rows;
             if (o.rows > 0) {
                 out = o;
                 return true;
             }
         }
-        // Deferred rows of resident partitions, by their resident tables.
-        for (; deferred_part_ < nparts_; deferred_part_++, deferred_chunk_ = 0) {
-            Part &P = parts_[deferred_part_];
-            while (!P.spilled && deferred_chunk_ < P.deferred.size()) {
-                DevBatch o = P.join->probe(load_group(P.deferred, deferred_chunk_));
-                counters_.output_rows += o.rows;
-                if (o.rows > 0) {
-                    out = o;
-                    return true;
-                }
-            }
-            P.join.reset();  // this resident table is done
-        }
+        for (Part &P : parts_) P.join.reset();
         for (;;) {
             if (fb_.active) {
                 if (fallback_next(out)) return true;
@@ -692,9 +835,11 @@ class GraceJoin {
             }
             if (cur_join_) {
                 if (prefetch_.pending || cur_probe_ < cur_.probe_host.size()) {
-                    DevBatch pb = prefetch_.pending ? take_prefetch() : load_group(cur_.probe_host, cur_probe_);
+                    if (!prefetch_.pending) start(prefetch_, cur_.probe_host, cur_probe_);
+                    DevBatch pb = take(prefetch_);
                     // the next group crosses the host link while this one is probed
-                    if (cur_probe_ < cur_.probe_host.size()) start_prefetch(cur_.probe_host, cur_probe_);
+                    if (cur_probe_ < cur_.probe_host.size()) start(prefetch_, cur_.probe_host, cur_probe_);
+                    else start_next_build();
                     DevBatch o = cur_join_->probe(pb);
                     counters_.output_rows += o.rows;
                     if (o.rows == 0) continue;
@@ -722,19 +867,23 @@ class GraceJoin {
             krv_join_spec js = spec_;
             js.build_rows_hint = rows;
             cur_join_.reset(new HashJoin(rt_, js));
+            if (rows && !next_build_.pending) start(next_build_, t.build_host, build_types_);
+            cur_ = std::move(t);
+            cur_rows_ = rows;
+            cur_probe_ = 0;
+            // the first probe rows cross the host link while the table is built
+            start(prefetch_, cur_.probe_host, cur_probe_);
             if (rows == 0) cur_join_->build_push(empty_like(build_types_));
-            else cur_join_->build_adopt(load_all(t.build_host, build_types_));
+            else cur_join_->build_adopt(take(next_build_));
             cur_join_->build_finish();
             counters_.build_keys += cur_join_->counters().build_keys;
             counters_.table_slots += cur_join_->counters().table_slots;
-            cur_ = std::move(t);
-            cur_probe_ = 0;
         }
     }
 
     bool done() const {
-        return finishing_ && pad_chunk_ >= pad_later_.size() && deferred_part_ >= nparts_ && !cur_join_ &&
-               tasks_.empty() && !fb_.active;
+        return finishing_ && !later_.pending && pad_chunk_ >= pad_later_.size() && deferred_part_ >= nparts_ &&
+               !cur_join_ && tasks_.empty() && !fb_.active;
     }
     // A zero-row batch of the output's shape.
     DevBatch empty_output() {
@@ -854,23 +1003,23 @@ class GraceJoin {
             if (victim < 0) break;
             Part &P = parts_[victim];
             if (P.build_rows > 0) {
-                Segment s;
-                s.batch = P.join->staged();
-                s.rows = P.build_rows;
-                P.build_host.push_back(spill(s));
+                const DevBatch b = P.join->staged();
+                Rows r;
+                r.add(victim, P.build_rows);
+                for (const DevCol &c : b.cols) r.cols.push_back(c.hold_data);
+                P.build_host.push_back(spill(r, build_types_)[0]);
             }
             P.join.reset();
             P.spilled = true;
         }
     }
 
-    // Partitions batch `b` by its key column at `level`: one segment (a
-    // device batch of the partition's rows) per partition, plus the NULL-key
-    // bucket at index nparts (kept when keep_nulls).
-    std::vector<Segment> partition(const DevBatch &b, int key, int level, int bits, bool keep_nulls,
-                                   int filter_mode = kFilterNone) {
+    // Counts the rows of `b` by bucket: the partitions of its key column at
+    // `level`, the NULL keys, the rows the filter rules out.
+    Counted count(const DevBatch &b, int key, int level, int bits, bool keep_nulls, int filter_mode = kFilterNone) {
         const int nparts = level == 0 ? (1 << bits) : 8;
-        PartArgs A{};
+        Counted k;
+        PartArgs &A = k.args;
         A.key = static_cast<const long long *>(b.cols[key].data);
         A.kvalid = b.cols[key].valid;
         A.kvoff = b.cols[key].valid_off;
@@ -885,74 +1034,59 @@ class GraceJoin {
         A.bloom = bloom_ ? bloom_->as<uint32_t>() : nullptr;
         A.bloom_blocks = bloom_blocks_;
         A.ncols = (int)b.cols.size();
+        for (int c = 0; c < A.ncols; c++) A.c[c] = PartCol{b.cols[c].data, nullptr, b.cols[c].type.width()};
         const int nb = nparts + 2;  // partitions, the NULL bucket, the filtered bucket
-        DBuf ctr(rt_, (size_t)nb * 8 * 2);
-        DBuf bucket;
+        k.ctr = DBuf(rt_, (size_t)nb * 8 * 2);
         if (filter_mode == kFilterTest && b.rows > 0) {
-            bucket = DBuf(rt_, (size_t)b.rows);
-            A.bucket = bucket.as<uint8_t>();
+            k.bucket = DBuf(rt_, (size_t)b.rows);
+            A.bucket = k.bucket.as<uint8_t>();
         }
-        unsigned long long *hist = ctr.as<unsigned long long>(), *cursor = hist + nb;
-        KRV_CUDA(cudaMemsetAsync(hist, 0, (size_t)nb * 8, rt_->stream));
-        part_hist_kernel<<<grid_for(rt_, b.rows, 256, 8), 256, 0, rt_->stream>>>(A, hist);
+        KRV_CUDA(cudaMemsetAsync(k.ctr.get(), 0, (size_t)nb * 8 * 2, rt_->stream));  // and the scatter's cursors
+        part_hist_kernel<<<grid_for(rt_, b.rows, 256, 8), 256, 0, rt_->stream>>>(A, k.ctr.as<unsigned long long>());
         rt_->launches++;
         check_launch("part_hist_kernel");
-        std::vector<unsigned long long> h(nb);
-        KRV_CUDA(cudaMemcpyAsync(h.data(), hist, nb * 8, cudaMemcpyDeviceToHost, rt_->stream));
-        KRV_CUDA(cudaStreamSynchronize(rt_->stream));
-        last_filtered_ = (int64_t)h[nparts + 1];  // counted whether the bucket is kept or dropped
-        std::vector<unsigned long long> start(nb);
-        std::vector<bool> kept_bucket(nb, true);
-        kept_bucket[nparts] = keep_nulls;
-        kept_bucket[nparts + 1] = A.keep_filtered != 0;
-        unsigned long long acc = 0;
-        for (int p = 0; p < nb; p++) {
-            start[p] = acc;
-            if (kept_bucket[p]) acc += h[p];
-        }
-        KRV_CUDA(cudaMemcpyAsync(cursor, start.data(), nb * 8, cudaMemcpyHostToDevice, rt_->stream));
-        const int64_t kept = (int64_t)acc;
-        std::vector<std::shared_ptr<DBuf>> outs;
-        for (int c = 0; c < A.ncols; c++) {
-            const int w = b.cols[c].type.width();
-            outs.push_back(std::make_shared<DBuf>(rt_, (size_t)std::max<int64_t>(kept, 1) * w));
-            A.c[c] = PartCol{b.cols[c].data, outs.back()->get(), w};
-        }
-        if (kept > 0) {
-            part_scatter_kernel<<<grid_for(rt_, ceil_div(b.rows, kPartTile), 1, 4), kPartThreads, 0, rt_->stream>>>(
-                A, cursor);
-            rt_->launches++;
-            check_launch("part_scatter_kernel");
-        }
-        std::vector<Segment> segs(nb);
-        for (int p = 0; p < nb; p++) {
-            Segment &s = segs[p];
-            s.rows = kept_bucket[p] ? (int64_t)h[p] : 0;
-            s.batch.rows = s.rows;
-            for (int c = 0; c < A.ncols; c++) {
-                DevCol col;
-                col.type = b.cols[c].type;
-                col.name = b.cols[c].name;
-                col.nullable = b.cols[c].nullable;
-                col.length = s.rows;
-                col.hold_data = outs[c];
-                col.data = outs[c]->as<uint8_t>() + start[p] * (size_t)b.cols[c].type.width();
-                s.batch.cols.push_back(col);
-            }
-        }
-        return segs;
+        k.rows.resize(nb);
+        read_device(rt_, k.ctr.get(), (size_t)nb * 8, k.rows.data());
+        return k;
     }
 
-    // The NULL bucket's rows with their key column marked NULL.
-    DevBatch with_null_keys(const Segment &s) {
-        DevBatch b = s.batch;
-        const int key = spec_.probe_keys[0];
-        auto bits = std::make_shared<DBuf>(rt_, (size_t)ceil_div(s.rows, 8) + 8);
-        KRV_CUDA(cudaMemsetAsync(bits->get(), 0, bits->bytes(), rt_->stream));
-        b.cols[key].hold_valid = bits;
-        b.cols[key].valid = bits->as<uint8_t>();
-        b.cols[key].valid_off = 0;
-        b.cols[key].nullable = true;
+    // Buffers for the rows of `r`, and their place in the scatter's table.
+    void place(Rows &r, const std::vector<DevCol> &types, const Counted &k, std::vector<void *> &to) {
+        if (r.rows == 0) return;
+        const size_t nb = k.rows.size();
+        for (size_t c = 0; c < types.size(); c++) {
+            const size_t w = (size_t)types[c].type.width();
+            r.cols.push_back(std::make_shared<DBuf>(rt_, (size_t)r.rows * w));
+            uint8_t *p = r.cols.back()->as<uint8_t>();
+            for (const auto &run : r.runs) {
+                to[c * nb + run.first] = p;
+                p += (size_t)run.second * w;
+            }
+        }
+    }
+    void scatter(Counted &k, const std::vector<void *> &to) {
+        if (std::all_of(to.begin(), to.end(), [](void *p) { return p == nullptr; })) return;  // no row is kept
+        k.to = DBuf(rt_, to.size() * sizeof(void *));
+        KRV_CUDA(cudaMemcpyAsync(k.to.get(), to.data(), to.size() * sizeof(void *), cudaMemcpyHostToDevice, rt_->stream));
+        k.args.to = k.to.as<void *>();
+        part_scatter_kernel<<<grid_for(rt_, ceil_div(k.args.n, kPartTile), 1, 4), kPartThreads, 0, rt_->stream>>>(
+            k.args, k.ctr.as<unsigned long long>() + k.rows.size());
+        rt_->launches++;
+        check_launch("part_scatter_kernel");
+    }
+    static DevBatch batch_of(const Rows &r, const std::vector<DevCol> &types) {
+        DevBatch b;
+        b.rows = r.rows;
+        for (size_t c = 0; c < types.size(); c++) {
+            DevCol col;
+            col.type = types[c].type;
+            col.name = types[c].name;
+            col.nullable = types[c].nullable;
+            col.length = r.rows;
+            col.hold_data = r.cols[c];
+            col.data = r.cols[c]->get();
+            b.cols.push_back(col);
+        }
         return b;
     }
 
@@ -984,32 +1118,34 @@ class GraceJoin {
         return p;
     }
 
-    // Copies a segment to the spill space (asynchronously, stream-ordered).
-    // Copies a segment to the spill space on the copy stream, so that the
-    // transfer overlaps the next slice's kernels; the segment's device
-    // buffers stay alive until the copy has landed.
-    HostChunk spill(const Segment &s) {
-        HostChunk h;
-        h.rows = s.rows;
+    // Copies rows to the spill space on the copy stream, one copy per column,
+    // so that the transfer overlaps the next slice's kernels; the device
+    // buffers stay alive until the copy has landed. One chunk per run.
+    std::vector<HostChunk> spill(const Rows &s, const std::vector<DevCol> &types) {
+        std::vector<HostChunk> h(s.runs.size());
+        if (s.rows == 0) return h;
         cudaEvent_t ready;
         KRV_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
         KRV_CUDA(cudaEventRecord(ready, rt_->stream));
         KRV_CUDA(cudaStreamWaitEvent(cs_, ready, 0));
         KRV_CUDA(cudaEventDestroy(ready));
         InFlight f;
-        for (const DevCol &c : s.batch.cols) {
-            const size_t bytes = (size_t)s.rows * c.type.width();
+        for (size_t c = 0; c < types.size(); c++) {
+            const size_t w = (size_t)types[c].type.width(), bytes = (size_t)s.rows * w;
             uint8_t *p = host_alloc(bytes);
-            KRV_CUDA(cudaMemcpyAsync(p, c.data, bytes, cudaMemcpyDeviceToHost, cs_));
-            h.cols.push_back(p);
-            f.hold.push_back(c.hold_data);
+            KRV_CUDA(cudaMemcpyAsync(p, s.cols[c]->get(), bytes, cudaMemcpyDeviceToHost, cs_));
+            for (size_t i = 0; i < s.runs.size(); i++) {
+                h[i].rows = s.runs[i].second;
+                h[i].cols.push_back(p);
+                p += (size_t)s.runs[i].second * w;
+            }
+            f.hold.push_back(s.cols[c]);
             f.bytes += bytes;
         }
         KRV_CUDA(cudaEventCreateWithFlags(&f.done, cudaEventDisableTiming));
         KRV_CUDA(cudaEventRecord(f.done, cs_));
         inflight_bytes_ += f.bytes;
         inflight_.push_back(std::move(f));
-        spilled_bytes_ += (int64_t)s.rows * row_bytes_;
         reap(false);
         // A short queue of spills: other small transfers share the copy engines.
         while (inflight_bytes_ > std::min<size_t>((size_t)(budget_ / 8), (size_t)1 << 30) && !inflight_.empty())
@@ -1039,31 +1175,70 @@ class GraceJoin {
     }
 
     // The probe chunks from `at` on that fit one slice, copied to the device on
-    // the copy stream; take_prefetch orders the join's stream after them.
-    void start_prefetch(const std::vector<HostChunk> &hs, size_t &at) {
+    // the copy stream (after the spills that may still be on their way); take
+    // orders the join's stream after them.
+    struct Prefetch {
+        DevBatch batch;
+        DBuf table;
+        cudaEvent_t ready = nullptr;
+        bool pending = false;
+    };
+    void start(Prefetch &f, const std::vector<HostChunk> &hs, size_t &at) {
         std::vector<HostChunk> group;
         int64_t rows = 0;
         while (at < hs.size() && (group.empty() || rows + hs[at].rows <= slice_rows())) {
             rows += hs[at].rows;
             group.push_back(hs[at++]);
         }
-        prefetch_.batch = alloc_like(probe_types_, rows);  // allocated in the join's stream order
+        start(f, group, probe_types_);
+    }
+    void start(Prefetch &f, const std::vector<HostChunk> &group, const std::vector<DevCol> &types) {
+        int64_t rows = 0;
+        for (const HostChunk &h : group) rows += h.rows;
+        f.batch = alloc_like(types, rows);  // allocated in the join's stream order
+        f.table = DBuf(rt_, group.size() * f.batch.cols.size() * sizeof(GatherRun));
         cudaEvent_t ready;
         KRV_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
         KRV_CUDA(cudaEventRecord(ready, rt_->stream));
         KRV_CUDA(cudaStreamWaitEvent(cs_, ready, 0));
         KRV_CUDA(cudaEventDestroy(ready));
-        copy_in(group, prefetch_.batch, cs_);
-        if (!prefetch_.ready) KRV_CUDA(cudaEventCreateWithFlags(&prefetch_.ready, cudaEventDisableTiming));
-        KRV_CUDA(cudaEventRecord(prefetch_.ready, cs_));
-        prefetch_.pending = true;
+        copy_in(group, f.batch, f.table, cs_);
+        if (!f.ready) KRV_CUDA(cudaEventCreateWithFlags(&f.ready, cudaEventDisableTiming));
+        KRV_CUDA(cudaEventRecord(f.ready, cs_));
+        f.pending = true;
     }
-    DevBatch take_prefetch() {
-        KRV_CUDA(cudaStreamWaitEvent(rt_->stream, prefetch_.ready, 0));
-        prefetch_.pending = false;
-        DevBatch b = std::move(prefetch_.batch);
-        prefetch_.batch = DevBatch{};
+    DevBatch take(Prefetch &f) {
+        KRV_CUDA(cudaStreamWaitEvent(rt_->stream, f.ready, 0));
+        f.pending = false;
+        DevBatch b = std::move(f.batch);
+        f.batch = DevBatch{};
         return b;
+    }
+    // The next spilled partition's build rows, while the last probe rows of
+    // the current one are joined, if both tables fit the resident share.
+    void start_next_build() {
+        if (next_build_.pending || tasks_.empty() || tasks_.front().probe_host.empty()) return;
+        int64_t rows = 0;
+        for (const HostChunk &c : tasks_.front().build_host) rows += c.rows;
+        if (rows == 0 || est_part_bytes(cur_rows_) + est_part_bytes(rows) > resident_cap()) return;
+        start(next_build_, tasks_.front().build_host, build_types_);
+    }
+    // The next rows put off by the probe calls: ruled-out ones (later_part_
+    // -1), then a resident partition's. False when none is left.
+    bool start_later() {
+        if (pad_chunk_ < pad_later_.size()) {
+            later_part_ = -1;
+            start(later_, pad_later_, pad_chunk_);
+            return true;
+        }
+        for (; deferred_part_ < nparts_; deferred_part_++, deferred_chunk_ = 0) {
+            const Part &P = parts_[deferred_part_];
+            if (P.spilled || deferred_chunk_ >= P.deferred.size()) continue;
+            later_part_ = deferred_part_;
+            start(later_, P.deferred, deferred_chunk_);
+            return true;
+        }
+        return false;
     }
     DevBatch alloc_like(const std::vector<DevCol> &types, int64_t rows) {
         DevBatch b;
@@ -1080,29 +1255,27 @@ class GraceJoin {
         }
         return b;
     }
-    void copy_in(const std::vector<HostChunk> &hs, DevBatch &b, cudaStream_t st) {
+    // The chunks' rows into `b`, in `st`'s order (the table is allocated and
+    // freed in the join's stream's, which `st` has waited for and which waits
+    // for `st` before it goes on).
+    void copy_in(const std::vector<HostChunk> &hs, DevBatch &b, DBuf &table, cudaStream_t st) {
+        std::vector<GatherRun> runs;
+        int64_t tiles = 0;
         for (size_t c = 0; c < b.cols.size(); c++) {
             const int w = b.cols[c].type.width();
             int64_t at = 0;
             for (const HostChunk &h : hs) {
-                if (h.rows)
-                    KRV_CUDA(cudaMemcpyAsync(b.cols[c].hold_data->as<uint8_t>() + at * w, h.cols[c], (size_t)h.rows * w,
-                                             cudaMemcpyHostToDevice, st));
+                if (h.rows == 0) continue;
+                runs.push_back(GatherRun{h.cols[c], b.cols[c].hold_data->as<uint8_t>() + at * w, h.rows, w, 0, tiles});
+                tiles += ceil_div(h.rows, (int64_t)kGatherThreads * kGatherWords);
                 at += h.rows;
             }
         }
-    }
-
-    // Probe chunks from `at` on, as many as fit one slice, loaded as one
-    // device batch; `at` moves past them.
-    DevBatch load_group(const std::vector<HostChunk> &hs, size_t &at) {
-        std::vector<HostChunk> group;
-        int64_t rows = 0;
-        while (at < hs.size() && (group.empty() || rows + hs[at].rows <= slice_rows())) {
-            rows += hs[at].rows;
-            group.push_back(hs[at++]);
-        }
-        return load_all(group, probe_types_);
+        if (runs.empty()) return;
+        KRV_CUDA(cudaMemcpyAsync(table.get(), runs.data(), runs.size() * sizeof(GatherRun), cudaMemcpyHostToDevice, st));
+        gather_kernel<<<(int)std::min<int64_t>(tiles, kGatherBlocks), kGatherThreads, 0, st>>>(table.as<GatherRun>(), (int)runs.size(), tiles);
+        rt_->launches++;
+        check_launch("gather_kernel");
     }
 
     DevBatch load(const HostChunk &h, const std::vector<DevCol> &types) {
@@ -1116,7 +1289,8 @@ class GraceJoin {
         for (const HostChunk &h : hs) rows += h.rows;
         if (!inflight_.empty()) KRV_CUDA(cudaStreamWaitEvent(rt_->stream, inflight_.back().done, 0));
         DevBatch b = alloc_like(types, rows);
-        copy_in(hs, b, rt_->stream);
+        DBuf table(rt_, hs.size() * b.cols.size() * sizeof(GatherRun));
+        copy_in(hs, b, table, rt_->stream);
         return b;
     }
 
@@ -1289,21 +1463,28 @@ class GraceJoin {
         return true;
     }
 
+    void split_side(const std::vector<HostChunk> &from, const std::vector<DevCol> &types, int key, int level,
+                    std::vector<Task> &sub, std::vector<HostChunk> Task::*side) {
+        for (const HostChunk &h : from) {
+            const DevBatch b = load(h, types);
+            Counted k = count(b, key, level, 3, false);
+            std::vector<void *> to(k.args.ncols * k.rows.size(), nullptr);
+            Rows host;
+            for (int p = 0; p < 8; p++) host.add(p, (int64_t)k.rows[p]);
+            place(host, types, k, to);
+            scatter(k, to);
+            const std::vector<HostChunk> chunks = spill(host, types);
+            for (size_t i = 0; i < chunks.size(); i++) (sub[host.runs[i].first].*side).push_back(chunks[i]);
+        }
+    }
+
     // Splits task `t` 8 ways with the next level of hash bits, chunk by chunk.
     void split(Task &t) {
         const int level = t.level + 1;
         std::vector<Task> sub(8);
         for (auto &s : sub) s.level = level;
-        for (const HostChunk &h : t.build_host) {
-            std::vector<Segment> segs = partition(load(h, build_types_), spec_.build_keys[0], level, 3, false);
-            for (int p = 0; p < 8; p++)
-                if (segs[p].rows) sub[p].build_host.push_back(spill(segs[p]));
-        }
-        for (const HostChunk &h : t.probe_host) {
-            std::vector<Segment> segs = partition(load(h, probe_types_), spec_.probe_keys[0], level, 3, false);
-            for (int p = 0; p < 8; p++)
-                if (segs[p].rows) sub[p].probe_host.push_back(spill(segs[p]));
-        }
+        split_side(t.build_host, build_types_, spec_.build_keys[0], level, sub, &Task::build_host);
+        split_side(t.probe_host, probe_types_, spec_.probe_keys[0], level, sub, &Task::probe_host);
         splits_ += 8;
         for (auto &s : sub) tasks_.push_front(std::move(s));
     }
@@ -1316,7 +1497,6 @@ class GraceJoin {
     int64_t bloom_bytes_ = 0;
     uint64_t bloom_blocks_ = 0;
     int64_t counters_filtered_ = 0;
-    int64_t last_filtered_ = 0;  // rows the last partition pass's filter ruled out
     std::vector<HostChunk> pad_later_;  // ruled-out probe rows past a call's output share (left outer)
     size_t pad_chunk_ = 0;
     bool schema_ = false, built_ = false, finishing_ = false;
@@ -1325,11 +1505,11 @@ class GraceJoin {
     int parts_bits_ = 3, nparts_ = 0;
     int64_t splits_ = 0;
     std::vector<Part> parts_;
-    int64_t spilled_bytes_ = 0;
     std::unique_ptr<HashJoin> null_join_;
     std::deque<Task> tasks_;
     Task cur_;
     size_t cur_probe_ = 0;
+    int64_t cur_rows_ = 0;
     int deferred_part_ = 0;
     size_t deferred_chunk_ = 0;
     std::unique_ptr<HashJoin> cur_join_;
@@ -1343,11 +1523,11 @@ class GraceJoin {
     };
     std::deque<InFlight> inflight_;
     size_t inflight_bytes_ = 0;
-    struct Prefetch {
-        DevBatch batch;
-        cudaEvent_t ready = nullptr;
-        bool pending = false;
-    } prefetch_;
+    Prefetch prefetch_, later_, next_build_;
+    int later_part_ = -1;
+    // The NULL build columns of padded rows
+    std::shared_ptr<DBuf> null_data_, null_valid_;
+    int64_t null_rows_ = 0;
     uint8_t *cur_block_ = nullptr;
     size_t cur_block_used_ = 0;
     krv_join_counters counters_{};

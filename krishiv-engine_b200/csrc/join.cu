@@ -1048,24 +1048,8 @@ HashJoin::HashJoin(Runtime *rt, const krv_join_spec &spec) : rt_(rt), spec_(spec
     counters_.partitions = 1;
 }
 
-void HashJoin::append_arena(const DevBatch &b) {
-    if (!have_schema_) {
-        for (const DevCol &c : b.cols) {
-            DevCol a;
-            a.type = c.type;
-            a.name = c.name;
-            a.nullable = c.nullable;
-            arena_cols_.push_back(a);
-        }
-        arena_data_.resize(b.cols.size());
-        arena_valid_.resize(b.cols.size());
-        have_schema_ = true;
-    } else {
-        if (b.cols.size() != arena_cols_.size()) fail(KRV_INVALID_ARGUMENT, "build batches differ in columns");
-        for (size_t i = 0; i < b.cols.size(); i++)
-            if (b.cols[i].type != arena_cols_[i].type) fail(KRV_INVALID_ARGUMENT, "build batches differ in types");
-    }
-    const int64_t need = build_rows_ + b.rows;
+// Room for `need` build rows in the arena.
+void HashJoin::grow_arena(int64_t need) {
     if (need > (int64_t)0xFFFFFFFEll) fail(KRV_UNSUPPORTED, "more than 2^32-2 build rows in one table");
     if (need > arena_cap_) {
         int64_t cap = std::max<int64_t>({need, arena_cap_ * 2, spec_.build_rows_hint, 1024});
@@ -1102,6 +1086,46 @@ void HashJoin::append_arena(const DevBatch &b) {
         }
         arena_cap_ = cap;
     }
+}
+
+// Room for `rows` more build rows (no NULLs), which the caller's kernels
+// write: where each column's begin. They count from build_commit on.
+void HashJoin::build_reserve(int64_t rows, void **dst) {
+    if (built_ || !have_schema_ || coded_) fail(KRV_INTERNAL, "build_reserve takes a plain build side's rows");
+    DeviceGuard g(rt_);
+    grow_arena(build_rows_ + rows);
+    for (size_t i = 0; i < arena_cols_.size(); i++) {
+        const DType t = arena_cols_[i].type;
+        if (t.id == Type::Bool || t.var()) fail(KRV_UNSUPPORTED, "build_reserve takes fixed-width columns");
+        dst[i] = arena_data_[i]->as<uint8_t>() + (size_t)build_rows_ * t.width();
+    }
+}
+
+void HashJoin::build_commit(int64_t rows) {
+    for (size_t i = 0; i < arena_cols_.size(); i++)
+        if (arena_valid_[i]) set_bits(rt_, arena_valid_[i]->as<uint8_t>(), build_rows_, rows);
+    build_rows_ += rows;
+}
+
+void HashJoin::append_arena(const DevBatch &b) {
+    if (!have_schema_) {
+        for (const DevCol &c : b.cols) {
+            DevCol a;
+            a.type = c.type;
+            a.name = c.name;
+            a.nullable = c.nullable;
+            arena_cols_.push_back(a);
+        }
+        arena_data_.resize(b.cols.size());
+        arena_valid_.resize(b.cols.size());
+        have_schema_ = true;
+    } else {
+        if (b.cols.size() != arena_cols_.size()) fail(KRV_INVALID_ARGUMENT, "build batches differ in columns");
+        for (size_t i = 0; i < b.cols.size(); i++)
+            if (b.cols[i].type != arena_cols_[i].type) fail(KRV_INVALID_ARGUMENT, "build batches differ in types");
+    }
+    const int64_t need = build_rows_ + b.rows;
+    grow_arena(need);
     for (size_t i = 0; i < arena_cols_.size(); i++) {
         const DevCol &c = b.cols[i];
         const DType t = c.type;

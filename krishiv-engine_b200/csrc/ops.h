@@ -131,6 +131,9 @@ class HashJoin {
     // Takes a batch whose columns own their device memory as the whole build
     // side, without copying (one batch, before any push).
     void build_adopt(DevBatch b);
+    // Build rows written in place by the caller's kernels.
+    void build_reserve(int64_t rows, void **dst);
+    void build_commit(int64_t rows);
     void build_finish();
     // Joins one probe batch; returns the output batch (all rows of it).
     DevBatch probe(const DevBatch &in);
@@ -183,6 +186,7 @@ class HashJoin {
 
   private:
     void append_arena(const DevBatch &b);
+    void grow_arena(int64_t need);
     // String or binary join keys: the key dictionary codes each key tuple as
     // one int64 (the build side inserts, the probe side looks up, -1 for a
     // key the build never saw); the table and kernels then join on that code.
