@@ -143,15 +143,25 @@ __global__ void fill_u64_kernel(unsigned long long *p, uint64_t n, unsigned long
 // RuntimeBloom::insert_hash (bloom.rs:136-148) for every kept key.
 __global__ void __launch_bounds__(256) bloom_insert_kernel(const int64_t *keys, const uint8_t *valid, int64_t voff,
                                                            int64_t n, uint32_t *words, uint64_t nblocks) {
-    // Eight lanes per key, lane w setting the key's bit in word w: a warp's
-    // atomic instruction then touches 4 blocks (one 32-byte sector each)
-    // instead of 32.
-    const int w = (int)(threadIdx.x & 7u);
-    const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 3;
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; i < n; i += stride) {
-        if (!bit_get(valid, voff, i)) continue;
-        const uint64_t h = xxh64_u64((uint64_t)keys[i]);
-        atomicOr(words + sbbf_block(h, nblocks) * 8 + w, sbbf_bit((uint32_t)h, w));
+    // A lane hashes one key; then the warp takes its 32 keys four at a time,
+    // eight lanes to a key, lane w of them setting the key's bit in word w: a
+    // warp's atomic instruction touches 4 blocks (one 32-byte sector each)
+    // instead of 32. Measured on B200, 1M keys: 18 us; 39 us with each
+    // key hashed by its eight lanes.
+    const int lane = lane_id(), w = lane & 7, q = lane >> 3;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); b < n; b += stride) {
+        const int64_t i = b + lane;
+        const bool live = i < n && bit_get(valid, voff, i);
+        const uint64_t h = live ? xxh64_u64((uint64_t)keys[i]) : 0;
+        const uint32_t block = (uint32_t)sbbf_block(h, nblocks);
+        const unsigned mask = __ballot_sync(0xFFFFFFFFu, live);
+#pragma unroll
+        for (int s = 0; s < 8; s++) {
+            const int src = s * 4 + q;
+            const uint32_t lo = __shfl_sync(0xFFFFFFFFu, (uint32_t)h, src), blk = __shfl_sync(0xFFFFFFFFu, block, src);
+            if ((mask >> src) & 1u) atomicOr(words + (uint64_t)blk * 8 + w, sbbf_bit(lo, w));
+        }
     }
 }
 
@@ -288,7 +298,7 @@ void finish_bloom(Runtime *rt, const krv_key_filter_options &opt, const DevCol &
     KRV_CUDA(cudaMemsetAsync(f.bloom.get(), 0, (size_t)bytes, rt->stream));
     const int64_t n = keys.length;
     if (n > 0) {
-        bloom_insert_kernel<<<grid_for(rt, n * 8, 256, 8), 256, 0, rt->stream>>>(
+        bloom_insert_kernel<<<grid_for(rt, n, 256, 8), 256, 0, rt->stream>>>(
             static_cast<const int64_t *>(keys.data), keys.valid, keys.valid_off, n, f.bloom.as<uint32_t>(),
             (uint64_t)(bytes / kBlockBytes));
         rt->launches++;

@@ -47,7 +47,8 @@ constexpr long long kAttrEmpty = (long long)0x8080808080808080ULL;
 constexpr int kSelectSteps = 16;
 constexpr int kSelectThreads = 256;
 constexpr int kSelectTile = kSelectThreads * kSelectSteps;
-__global__ void __launch_bounds__(kSelectThreads) dim_select_kernel(const long long *key, const int32_t *pred,
+constexpr int kSelectBlocks = 4;  // resident blocks per SM
+__global__ void __launch_bounds__(kSelectThreads, kSelectBlocks) dim_select_kernel(const long long *key, const int32_t *pred,
                                                                     const int32_t *attr, int64_t n, int32_t value,
                                                                     long long *okey, int32_t *oattr,
                                                                     unsigned long long *count, long long *range,
@@ -56,17 +57,29 @@ __global__ void __launch_bounds__(kSelectThreads) dim_select_kernel(const long l
     __shared__ unsigned long long s_base;
     __shared__ long long s_rng[4][kSelectThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    long long lo = LLONG_MAX, hi = LLONG_MIN, alo = LLONG_MAX, ahi = LLONG_MIN;
+    long long lo = LLONG_MAX, hi = LLONG_MIN;
+    int32_t amin = INT32_MAX, amax = INT32_MIN;
+    // The next tile's predicates are loaded while this one's keys are (20M
+    // rows, 5% selected, on B200: 65 us, 74 without).
+    int32_t nxt[kSelectSteps];
+    auto predicates = [&](int64_t c0) {
+#pragma unroll
+        for (int s = 0; s < kSelectSteps; s++) {
+            const int64_t i = c0 + s * 32 + lane;
+            nxt[s] = pred && i < n ? __ldcs(pred + i) : value;
+        }
+    };
+    predicates((int64_t)blockIdx.x * kSelectTile + (int64_t)warp * 32 * kSelectSteps);
     for (int64_t t0 = (int64_t)blockIdx.x * kSelectTile; t0 < n; t0 += (int64_t)gridDim.x * kSelectTile) {
         const int64_t c0 = t0 + (int64_t)warp * 32 * kSelectSteps;
         unsigned ballots[kSelectSteps];
         unsigned total = 0;
 #pragma unroll
         for (int s = 0; s < kSelectSteps; s++) {
-            const int64_t i = c0 + s * 32 + lane;
-            ballots[s] = __ballot_sync(0xFFFFFFFFu, i < n && (!pred || pred[i] == value));
+            ballots[s] = __ballot_sync(0xFFFFFFFFu, c0 + s * 32 + lane < n && nxt[s] == value);
             total += __popc(ballots[s]);
         }
+        predicates(c0 + (int64_t)gridDim.x * kSelectTile);
         if (lane == 0) s_tot[warp] = total;
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -81,25 +94,25 @@ __global__ void __launch_bounds__(kSelectThreads) dim_select_kernel(const long l
         // The selected rows' keys and attributes, all loads issued before
         // any store (a load placed after a store to the output would wait
         // for it: the compiler cannot tell the arrays apart).
-        // Half the steps at a time, to stay within the registers.
-        constexpr int kHalf = kSelectSteps / 2;
+        // A quarter of the steps at a time, to stay within the registers.
+        constexpr int kPart = kSelectSteps / 4;
         __syncthreads();
         unsigned long long base = s_base + s_tot[warp];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            long long ks[kHalf];
-            int32_t as[kHalf];
+        for (int h = 0; h < 4; h++) {
+            long long ks[kPart];
+            int32_t as[kPart];
 #pragma unroll
-            for (int q = 0; q < kHalf; q++) {
-                const int s = h * kHalf + q;
+            for (int q = 0; q < kPart; q++) {
+                const int s = h * kPart + q;
                 const int64_t i = c0 + s * 32 + lane;
                 const bool mine = (ballots[s] >> lane) & 1u;
                 ks[q] = mine ? key[i] : 0;
                 as[q] = mine && attr ? attr[i] : 0;
             }
 #pragma unroll
-            for (int q = 0; q < kHalf; q++) {
-                const int s = h * kHalf + q;
+            for (int q = 0; q < kPart; q++) {
+                const int s = h * kPart + q;
                 if ((ballots[s] >> lane) & 1u) {
                     const unsigned long long pos = base + __popc(ballots[s] & lanemask_lt());
                     const long long k = ks[q];
@@ -108,8 +121,8 @@ __global__ void __launch_bounds__(kSelectThreads) dim_select_kernel(const long l
                     oattr[pos] = a;
                     lo = k < lo ? k : lo;
                     hi = k > hi ? k : hi;
-                    alo = a < alo ? a : alo;
-                    ahi = a > ahi ? a : ahi;
+                    amin = min(a, amin);
+                    amax = max(a, amax);
                 }
                 base += __popc(ballots[s]);
             }
@@ -117,6 +130,7 @@ __global__ void __launch_bounds__(kSelectThreads) dim_select_kernel(const long l
         __syncthreads();  // s_tot is rewritten by the next tile
     }
     if (!range && !arange) return;
+    long long alo = lo <= hi ? amin : LLONG_MAX, ahi = lo <= hi ? amax : LLONG_MIN;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, d));
@@ -412,7 +426,7 @@ class StarPipeline {
     // range. False (nothing kept) when a dimension does not qualify: the
     // join-table build runs.
     int select_grid(int64_t n) const {
-        return (int)std::max<int64_t>(1, std::min<int64_t>(8 * rt_->sm_count, ceil_div(n, kSelectTile)));
+        return (int)std::max<int64_t>(1, std::min<int64_t>(kSelectBlocks * rt_->sm_count, ceil_div(n, kSelectTile)));
     }
     bool build_fast(const DevBatch *dims[2], const int32_t values[2]) {
         struct Sel {
