@@ -3,17 +3,18 @@
 // over build tables kept resident on the device, with requests admitted by an
 // HBM budget and run in ticks.
 //
-// Batched mode. A tick is one CUDA graph of three kernels over descriptors
-// uploaded before it: clear the accumulators of newly admitted requests; one
-// probe + aggregate launch over a device work queue of (request, row range)
-// items from every running request, CTAs taking items off an atomic cursor;
+// Batched mode. A tick is one CUDA graph of three or four kernels over
+// descriptors uploaded before it in one copy: clear the accumulators of newly
+// admitted requests; a probe + aggregate launch over a device work queue of
+// (request, row range) items from every running request, CTAs taking items off
+// an atomic cursor (a second launch when requests have some thousand groups);
 // and compaction of the groups of the requests that end in the tick. A tick
 // takes at most `tick_rows` probe rows, so a large request spans several
 // ticks while requests that arrive meanwhile join the next one and finish
 // early (continuous batching). Two ticks may be queued at once: the host
 // forms and uploads the next while the device runs the current one.
 // Aggregation runs in shared memory for requests with few groups (per-CTA
-// 128-bit partial sums merged once per item) and in global memory otherwise.
+// 96-bit partial sums merged once per item) and in global memory otherwise.
 // An online autotuner tries the candidate kernel shapes (block size, item
 // rows, shared-memory group limit) on the first ticks and keeps the fastest.
 //
@@ -27,6 +28,7 @@
 // 314-330).
 #include <algorithm>
 #include <chrono>
+#include <cstring>
 #include <deque>
 #include <map>
 #include <memory>
@@ -43,7 +45,26 @@ namespace {
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
 constexpr int kMaxTickRequests = 512;
 constexpr int kMaxTickItems = 16384;
-constexpr int kSmemGroupsMax = 2048;  // shared-memory aggregation limit (48 KiB)
+constexpr int kTickRowsPerThread = 4;  // in flight together
+// Shared-memory aggregation: 16 bytes per group (see SmemGroups). The lookups
+// of a step are thousands of scattered reads, each holding a line of L1 while it
+// is on its way, and L1 is what shared memory leaves: so most requests run in
+// CTAs that leave three quarters of it (32 KB in each of two CTAs of 512
+// threads, or 16 KB in four of 256), and those with more groups, up to
+// kMidGroups, in a launch of their own with one CTA of 512 threads per SM.
+// Measured on B200, a tick of 38.5M rows of 24 requests with 10 to 68,000
+// groups: 0.41 ms; 0.68 with 7168 groups in each of two CTAs for all, 0.58 with
+// at most 2048 groups in shared memory, 0.45 with up to 12288 in the second
+// launch.
+constexpr int kSmemGroupBytes = 16;
+constexpr int tick_smem_groups(int threads) { return threads == 256 ? 1024 : 2048; }
+constexpr int kMidThreads = 512;
+constexpr int kMidGroups = 7168;
+// Requests of up to this many groups aggregate there however few rows an item
+// has, or (the autotuner's other choice, 0) only where the rows pay for it, as
+// all others do.
+constexpr int kSmemGroupsAlways = 2048;
+constexpr int kSmemRowsPerGroup = 4;
 constexpr unsigned long long kGroupEmpty = 0x8000000000000000ull;
 
 // How a resident table answers key -> group id:
@@ -81,13 +102,15 @@ struct ReqDev {
     int64_t kvoff;
     const long long *x;
     TableView t;
-    unsigned long long *lo;  // per group: 128-bit SUM (lo, hi) and COUNT(*)
+    unsigned long long *lo;  // per group: SUM (lo, hi) and COUNT(*)
     long long *hi;
     unsigned long long *cnt;
     const long long *gkeys;  // group value of each dense group id
     long long *out_g, *out_sum, *out_cnt;
     int32_t ngroups;
     int32_t use_smem;
+    int32_t split;   // SUM = hi * 2^32 + lo (at most 2^32 rows join); else 128 bits
+    int32_t copies;  // log2 of the copies of each group in shared memory
 };
 struct Item {
     int32_t req;
@@ -96,8 +119,9 @@ struct Item {
     int64_t rows;
 };
 struct TickHeader {
-    unsigned long long cursor;  // work queue cursor
-    int32_t n_items, n_init, n_final, pad;
+    unsigned long long cursor[2];  // of the two launches' work queues
+    int32_t n_items[2], items_at[2];  // the items follow the tick's requests: index (in Items) from TickDev::items
+    int32_t n_init, n_final;
 };
 struct Report {
     unsigned long long groups;
@@ -115,38 +139,76 @@ struct TickDev {
     Report *report;  // one per entry of `final`
 };
 
-__device__ __forceinline__ uint32_t table_head(const TableView &t, long long k) {
-    const uint64_t g = finalize(hash_word((uint64_t)k), t.seed);
-    const uint32_t tag = slot_tag(g);
-    uint64_t pos = g & t.mask;
-    for (uint64_t p = 0; p <= t.mask; p++) {
-        const unsigned long long s = __ldg(t.slots + pos);
-        if (s == 0) return kNoRow;
-        if (slot_matches(s, tag)) {
-            const uint32_t o = slot_row(s);
-            if (__ldg(t.keys + o) == k) return o;
+// The lookups of U rows (`has`: those with a key), their first reads in flight
+// together: from clamped addresses, without a branch before them.
+template <int U>
+__device__ __forceinline__ void table_heads(const TableView &t, const long long (&k)[U], unsigned has, uint32_t (&row)[U]) {
+    uint32_t tag[U];
+    uint64_t pos[U];
+    unsigned long long first[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint64_t g = finalize(hash_word((uint64_t)k[u]), t.seed);
+        tag[u] = slot_tag(g);
+        pos[u] = g & t.mask;
+        first[u] = __ldg(t.slots + pos[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        row[u] = kNoRow;
+        if (!((has >> u) & 1u)) continue;
+        unsigned long long s = first[u];
+        for (uint64_t p = 0; p <= t.mask && s != 0; p++) {
+            if (slot_matches(s, tag[u])) {
+                const uint32_t o = slot_row(s);
+                if (__ldg(t.keys + o) == k[u]) {
+                    row[u] = o;
+                    break;
+                }
+            }
+            pos[u] = (pos[u] + 1) & t.mask;
+            s = __ldg(t.slots + pos[u]);
         }
-        pos = (pos + 1) & t.mask;
     }
-    return kNoRow;
 }
 
-__device__ __forceinline__ int record_gid(const TableView &t, long long k) {
-    const uint64_t g = finalize(hash_word((uint64_t)k), t.seed);
-    uint64_t pos = g & t.mask;
-    for (uint64_t p = 0; p <= t.mask; p++) {
-        const longlong2 r = __ldg(reinterpret_cast<const longlong2 *>(t.rec + pos));
-        const int gid = (int)(int32_t)(r.y & 0xFFFFFFFFll);
-        if (gid < 0) return -1;
-        if (r.x == k) return gid;
-        pos = (pos + 1) & t.mask;
+template <int U>
+__device__ __forceinline__ void record_gids(const TableView &t, const long long (&k)[U], unsigned has, int (&g)[U]) {
+    uint64_t pos[U];
+    longlong2 first[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        pos[u] = finalize(hash_word((uint64_t)k[u]), t.seed) & t.mask;
+        first[u] = __ldg(reinterpret_cast<const longlong2 *>(t.rec + pos[u]));
     }
-    return -1;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        g[u] = -1;
+        if (!((has >> u) & 1u)) continue;
+        longlong2 r = first[u];
+        for (uint64_t p = 0; p <= t.mask; p++) {
+            const int gid = (int)(int32_t)(r.y & 0xFFFFFFFFll);
+            if (gid < 0) break;
+            if (r.x == k[u]) {
+                g[u] = gid;
+                break;
+            }
+            pos[u] = (pos[u] + 1) & t.mask;
+            r = __ldg(reinterpret_cast<const longlong2 *>(t.rec + pos[u]));
+        }
+    }
 }
 
-__device__ __forceinline__ int direct_gid(const TableView &t, long long k) {
-    const unsigned long long off = (unsigned long long)(k - t.lo);
-    return off <= t.span ? __ldg(t.direct + off) : -1;
+template <int U>
+__device__ __forceinline__ void direct_gids(const TableView &t, const long long (&k)[U], unsigned has, int (&g)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const unsigned long long off = (unsigned long long)(k[u] - t.lo);
+        g[u] = __ldg(t.direct + (off <= t.span ? off : 0ull));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        if (!((has >> u) & 1u) || (unsigned long long)(k[u] - t.lo) > t.span) g[u] = -1;
 }
 
 // Fills the records of a table with unique keys from its join slots.
@@ -169,128 +231,283 @@ __global__ void direct_kernel(const long long *keys, const int32_t *gid, int64_t
         direct[(unsigned long long)(keys[i] - lo)] = gid[i];
 }
 
-__global__ void tick_init_kernel(TickDev d) {
+// The groups of the requests listed in `list`, a chunk of kChunkGroups at a
+// time, spread over all CTAs: f(index into the list, request, first group).
+// (A loop over the requests waited for each one's descriptor in turn: 24
+// requests took 14 us to clear and 46 us to compact, now 3 and 10.)
+constexpr int kChunkThreads = 256;
+constexpr int kChunkGroups = 4 * kChunkThreads;
+template <class F> __device__ __forceinline__ void for_chunks(const TickDev &d, const int32_t *list, int n, F f) {
+    __shared__ int s_first[kMaxTickRequests + 1];  // each request's first chunk
+    __shared__ int s_warp[kChunkThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int before = 0;
+    for (int i0 = 0; i0 < n; i0 += kChunkThreads) {
+        const int i = i0 + threadIdx.x;
+        const int c = i < n ? (d.reqs[list[i]].ngroups + kChunkGroups - 1) / kChunkGroups : 0;
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int mine = before;
+        for (int w = 0; w < kChunkThreads / 32; w++) {
+            if (w < warp) mine += s_warp[w];
+            before += s_warp[w];
+        }
+        if (i < n) s_first[i] = mine + incl - c;
+        __syncthreads();
+    }
+    for (int c = blockIdx.x; c < before; c += gridDim.x) {
+        int lo = 0, hi = n - 1;  // the last request whose first chunk is at most c and that has one
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (s_first[mid] <= c) lo = mid;
+            else hi = mid - 1;
+        }
+        f(lo, d.reqs[list[lo]], (c - s_first[lo]) * kChunkGroups);
+    }
+}
+
+__global__ void __launch_bounds__(kChunkThreads) tick_init_kernel(TickDev d) {
     const TickHeader h = *d.hdr;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (int i = 0; i < h.n_init; i++) {
-        const ReqDev &r = d.reqs[d.init[i]];
-        for (int64_t gi = tid; gi < r.ngroups; gi += stride) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < h.n_final; i += gridDim.x * blockDim.x) d.report[i] = Report{0, 0, 0};
+    for_chunks(d, d.init, h.n_init, [&](int, const ReqDev &r, int g0) {
+        for (int gi = g0 + threadIdx.x; gi < min(g0 + kChunkGroups, r.ngroups); gi += kChunkThreads) {
             r.lo[gi] = 0;
             r.hi[gi] = 0;
             r.cnt[gi] = 0;
         }
-    }
-    for (int64_t i = tid; i < h.n_final; i += stride) d.report[i] = Report{0, 0, 0};
+    });
 }
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) tick_probe_kernel(TickDev d) {
+// ---- the groups' accumulators --------------------------------------------------
+// In device memory: SUM of a request whose joined rows cannot pass 2^32 is
+// kept as the sums of its values' low 32 bits and of their high parts, which
+// two atomics add without waiting for what they add to (the high part of a
+// small value is 0: none); otherwise as 128 bits, where the low word's old
+// value tells the carry.
+struct GroupSums {
+    unsigned long long *lo, *hi, *cnt;
+    bool split;
+    __device__ __forceinline__ void add(int g, long long x) const {
+        if (split) {
+            atomicAdd(lo + g, (unsigned long long)(uint32_t)x);
+            if (x >> 32) atomicAdd(hi + g, (unsigned long long)(x >> 32));
+        } else {
+            atomic_add_i128_from_i64(lo + g, reinterpret_cast<long long *>(hi) + g, x);
+        }
+        atomicAdd(cnt + g, 1ull);
+    }
+};
+// In shared memory: four 32-bit words per group and copy, word planes apart
+// (64-bit shared atomics are compare-and-swap loops, 32-bit ones are not): the
+// count, then SUM in 96 bits with its carries. Few groups have up to 32 copies,
+// one per lane, so that the lanes of a warp do not queue on one word.
+template <int CAP> struct SmemGroups {
+    uint32_t *w;
+    // `many`: more than 2^32 rows may join (duplicate build keys): the count's
+    // carries go straight to device memory.
+    __device__ __forceinline__ void add(int g, int copies, int copy, bool many, const GroupSums &G, long long x) const {
+        const int e = (g << copies) + copy;
+        if (!many) atomicAdd(w + e, 1u);
+        else if (atomicAdd(w + e, 1u) == 0xFFFFFFFFu) atomicAdd(G.cnt + g, 1ull << 32);
+        const uint32_t x0 = (uint32_t)x;
+        const uint32_t o0 = atomicAdd(w + CAP + e, x0);
+        const unsigned long long a1 = (unsigned long long)(uint32_t)(x >> 32) + (o0 + x0 < o0 ? 1u : 0u);
+        uint32_t a2 = (x < 0 ? 0xFFFFFFFFu : 0u) + (uint32_t)(a1 >> 32);
+        const uint32_t x1 = (uint32_t)a1;
+        if (x1) {
+            const uint32_t o1 = atomicAdd(w + 2 * CAP + e, x1);
+            a2 += o1 + x1 < o1 ? 1u : 0u;
+        }
+        if (a2) atomicAdd(w + 3 * CAP + e, a2);
+    }
+    __device__ __forceinline__ void clear(const ReqDev &R, int threads) const {
+        const int n = R.ngroups << R.copies;
+        for (int e = threadIdx.x; e < n; e += threads) {
+#pragma unroll
+            for (int p = 0; p < 4; p++) w[p * CAP + e] = 0;
+        }
+    }
+    // Adds the groups up and into device memory.
+    __device__ __forceinline__ void merge(const ReqDev &R, int threads) const {
+        for (int g = threadIdx.x; g < R.ngroups; g += threads) {
+            unsigned long long count = 0;
+            __int128 sum = 0;
+            for (int q = 0; q < (1 << R.copies); q++) {
+                const int e = (g << R.copies) + ((q + g) & ((1 << R.copies) - 1));
+                count += w[e];
+                sum += (__int128)(((unsigned long long)w[2 * CAP + e] << 32) | w[CAP + e]) +
+                       ((__int128)(long long)(int32_t)w[3 * CAP + e] << 64);
+            }
+            if (count) atomicAdd(R.cnt + g, count);
+            if (!sum) continue;
+            if (R.split) {
+                atomicAdd(R.lo + g, (unsigned long long)(uint32_t)sum);
+                atomicAdd(reinterpret_cast<unsigned long long *>(R.hi) + g, (unsigned long long)(long long)(sum >> 32));
+            } else {
+                atomic_add_i128(R.lo + g, R.hi + g, (int64_t)sum, (int64_t)(sum >> 64));
+            }
+        }
+    }
+};
+
+// One item's rows: U a thread and step, their loads in flight
+// together and the next step's keys and values loaded ahead. What a row needs of
+// its request is in registers, and no load stands behind a branch, where it
+// would be waited for by itself. Bound by the scattered lookups: the tick above
+// takes 0.15 ms without them, and 0.63 ms took it before (64-bit shared atomics,
+// the request's fields read again for every row, items of 32,768 rows).
+template <int THREADS, int U, int LAYOUT, bool SMEM, class S>
+__device__ __forceinline__ void item_rows(const ReqDev &R, const Item &it, const S &sums) {
+    const TableView T = R.t;
+    const GroupSums G{R.lo, reinterpret_cast<unsigned long long *>(R.hi), R.cnt, R.split != 0};
+    const int copies = R.copies, copy = (int)lane_id() & ((1 << copies) - 1);
+    const int64_t end = it.row0 + it.rows;
+    const long long *keys = R.k, *values = R.x;
+    const uint8_t *kvalid = R.kvalid;
+    const int64_t kvoff = R.kvoff;
+    auto add = [&](int g, long long x) {
+        if (SMEM) sums.add(g, copies, copy, LAYOUT == kChains, G, x);
+        else G.add(g, x);
+    };
+    long long k1[U], x1[U];  // the next step's rows
+    unsigned has1 = 0;
+    auto load = [&](int64_t base) {
+        has1 = 0;
+#pragma unroll
+        for (int u = 0; u < U; u++) {  // past the end: the last row again
+            const int64_t r = min(base + (int64_t)u * THREADS + threadIdx.x, end - 1);
+            k1[u] = __ldcs(keys + r);
+            x1[u] = __ldcs(values + r);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t r = base + (int64_t)u * THREADS + threadIdx.x;
+            if (r < end && (!kvalid || bit_get(kvalid, kvoff, r))) has1 |= 1u << u;
+        }
+    };
+    load(it.row0);
+    for (int64_t base = it.row0; base < end; base += (int64_t)THREADS * U) {
+        long long k[U], x[U];
+        const unsigned has = has1;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            k[u] = k1[u];
+            x[u] = x1[u];
+        }
+        load(base + (int64_t)THREADS * U);
+        if constexpr (LAYOUT == kChains) {
+            uint32_t row[U];
+            table_heads<U>(T, k, has, row);
+#pragma unroll
+            for (int u = 0; u < U; u++)  // every build row with this key (duplicates chain newest-first)
+                for (uint32_t b = row[u]; b != kNoRow; b = __ldg(T.next + b)) add(__ldg(T.gid + b), x[u]);
+        } else {
+            int g[U];
+            if constexpr (LAYOUT == kDirect) direct_gids<U>(T, k, has, g);
+            else record_gids<U>(T, k, has, g);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (g[u] >= 0) add(g[u], x[u]);
+        }
+    }
+}
+
+// QUEUE 0: the requests of few groups (in shared memory) or very many (in
+// device memory); 1: those between.
+template <int THREADS, int QUEUE>
+__global__ void __launch_bounds__(THREADS, QUEUE ? 1 : 1024 / THREADS) tick_probe_kernel(TickDev d) {
+    constexpr int U = kTickRowsPerThread;
     extern __shared__ __align__(16) uint8_t smem[];
-    unsigned long long *s_lo = reinterpret_cast<unsigned long long *>(smem);
-    long long *s_hi = reinterpret_cast<long long *>(s_lo + kSmemGroupsMax);
-    unsigned long long *s_cnt = reinterpret_cast<unsigned long long *>(s_hi + kSmemGroupsMax);
+    const SmemGroups<QUEUE ? kMidGroups : tick_smem_groups(THREADS)> S{reinterpret_cast<uint32_t *>(smem)};
     __shared__ int s_item;
-    const int n_items = d.hdr->n_items;
-    constexpr int U = 4;  // rows per thread in flight
+    const int n_items = d.hdr->n_items[QUEUE];
+    const Item *items = d.items + d.hdr->items_at[QUEUE];
     for (;;) {
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(&d.hdr->cursor, 1ull);
+        if (threadIdx.x == 0) s_item = (int)atomicAdd(&d.hdr->cursor[QUEUE], 1ull);
         __syncthreads();
         const int item = s_item;
-        __syncthreads();
         if (item >= n_items) break;
-        const Item it = d.items[item];
-        const ReqDev R = d.reqs[it.req];
-        const bool sm = R.use_smem != 0;
+        const Item it = items[n_items - 1 - item];
+        const ReqDev &R = d.reqs[it.req];
+        const bool sm = QUEUE || R.use_smem != 0;
+        if (sm) S.clear(R, THREADS);
+        __syncthreads();
         if (sm) {
-            for (int gi = threadIdx.x; gi < R.ngroups; gi += THREADS) {
-                s_lo[gi] = 0;
-                s_hi[gi] = 0;
-                s_cnt[gi] = 0;
-            }
-            __syncthreads();
+            if (R.t.layout == kDirect) item_rows<THREADS, U, kDirect, true>(R, it, S);
+            else if (R.t.layout == kRecords) item_rows<THREADS, U, kRecords, true>(R, it, S);
+            else item_rows<THREADS, U, kChains, true>(R, it, S);
+        } else if constexpr (QUEUE == 0) {
+            if (R.t.layout == kDirect) item_rows<THREADS, U, kDirect, false>(R, it, S);
+            else if (R.t.layout == kRecords) item_rows<THREADS, U, kRecords, false>(R, it, S);
+            else item_rows<THREADS, U, kChains, false>(R, it, S);
         }
-        const int64_t end = it.row0 + it.rows;
-        for (int64_t base = it.row0; base < end; base += (int64_t)THREADS * U) {
-            long long k[U], x[U];
-            bool has[U];
-            uint32_t row[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int64_t r = base + (int64_t)u * THREADS + threadIdx.x;
-                has[u] = r < end && (!R.kvalid || bit_get(R.kvalid, R.kvoff, r));
-                k[u] = has[u] ? __ldcs(R.k + r) : 0;
-                x[u] = has[u] ? __ldcs(R.x + r) : 0;
-            }
-            if (R.t.layout != kChains) {
-                int g[U];
-#pragma unroll
-                for (int u = 0; u < U; u++)
-                    g[u] = !has[u] ? -1 : R.t.layout == kDirect ? direct_gid(R.t, k[u]) : record_gid(R.t, k[u]);
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (g[u] < 0) continue;
-                    if (sm) {
-                        atomic_add_i128_from_i64(s_lo + g[u], s_hi + g[u], x[u]);
-                        atomicAdd(s_cnt + g[u], 1ull);
-                    } else {
-                        atomic_add_i128_from_i64(R.lo + g[u], R.hi + g[u], x[u]);
-                        atomicAdd(R.cnt + g[u], 1ull);
-                    }
-                }
-                continue;
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) row[u] = has[u] ? table_head(R.t, k[u]) : kNoRow;
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                // every build row with this key (duplicates chain newest-first)
-                for (uint32_t b = row[u]; b != kNoRow; b = __ldg(R.t.next + b)) {
-                    const int g = __ldg(R.t.gid + b);
-                    if (sm) {
-                        atomic_add_i128_from_i64(s_lo + g, s_hi + g, x[u]);
-                        atomicAdd(s_cnt + g, 1ull);
-                    } else {
-                        atomic_add_i128_from_i64(R.lo + g, R.hi + g, x[u]);
-                        atomicAdd(R.cnt + g, 1ull);
-                    }
-                }
-            }
-        }
+        __syncthreads();  // and s_item has been read by all
         if (sm) {
+            S.merge(R, THREADS);
             __syncthreads();
-            for (int gi = threadIdx.x; gi < R.ngroups; gi += THREADS) {
-                const unsigned long long c = s_cnt[gi];
-                if (!c) continue;
-                atomic_add_i128(R.lo + gi, R.hi + gi, (int64_t)s_lo[gi], s_hi[gi]);
-                atomicAdd(R.cnt + gi, c);
-            }
         }
     }
 }
 
 // The groups of each request that ends in this tick, compacted.
-__global__ void tick_final_kernel(TickDev d) {
+__global__ void __launch_bounds__(kChunkThreads) tick_final_kernel(TickDev d) {
     const TickHeader h = *d.hdr;
-    const unsigned active = 0xFFFFFFFFu;
-    for (int i = 0; i < h.n_final; i++) {
-        const ReqDev &r = d.reqs[d.final[i]];
-        const int64_t ng = r.ngroups;
-        const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-        const int64_t span = (ng + 31) / 32 * 32;  // whole warps
-        for (int64_t gi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gi < span; gi += stride) {
-            const bool in = gi < ng && r.cnt[gi] != 0;
-            const unsigned long long pos = warp_alloc(&d.report[i].groups, in, active);
-            if (!in) continue;
-            const unsigned long long l = r.lo[gi];
-            const long long hh = r.hi[gi];
-            const bool fits64 = (hh == 0 && !(l >> 63)) || (hh == -1 && (l >> 63));
-            if (!fits64) atomicOr(&d.report[i].overflow, 1u);
+    constexpr int U = kChunkGroups / kChunkThreads;
+    __shared__ unsigned s_warp[kChunkThreads / 32];
+    __shared__ unsigned long long s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for_chunks(d, d.final, h.n_final, [&](int i, const ReqDev &r, int g0) {
+        unsigned long long cnt[U];
+        int mine = 0;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int gi = g0 + u * kChunkThreads + threadIdx.x;
+            cnt[u] = gi < r.ngroups ? r.cnt[gi] : 0;
+            mine += cnt[u] != 0;
+        }
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_warp[warp] = (unsigned)incl;
+        __syncthreads();
+        unsigned at = 0, total = 0;
+        for (int w = 0; w < kChunkThreads / 32; w++) {
+            if (w < warp) at += s_warp[w];
+            total += s_warp[w];
+        }
+        if (threadIdx.x == 0) s_base = total ? atomicAdd(&d.report[i].groups, (unsigned long long)total) : 0ull;
+        __syncthreads();
+        unsigned long long pos = s_base + at + (unsigned)(incl - mine);
+        bool over = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!cnt[u]) continue;
+            const int gi = g0 + u * kChunkThreads + threadIdx.x;
+            unsigned long long l = r.lo[gi];
+            long long hh = r.hi[gi];
+            if (r.split) {
+                const __int128 sum = (__int128)hh * ((__int128)1 << 32) + (__int128)l;
+                l = (unsigned long long)sum;
+                hh = (long long)(sum >> 64);
+            }
+            over = over || !((hh == 0 && !(l >> 63)) || (hh == -1 && (l >> 63)));
             r.out_g[pos] = r.gkeys[gi];
             r.out_sum[pos] = (long long)l;
-            r.out_cnt[pos] = (long long)r.cnt[gi];
+            r.out_cnt[pos] = (long long)cnt[u];
+            pos++;
         }
-    }
+        if (over) atomicOr(&d.report[i].overflow, 1u);
+        __syncthreads();  // s_warp and s_base are written by the next chunk
+    });
 }
 
 // ---- the group directory of a resident table ------------------------------------
@@ -621,11 +838,12 @@ class Server {
             off = (off + bytes + 255) / 256 * 256;
             return base + o;
         };
+        // what a tick uses lies together, so that one copy uploads it
         uint8_t *hdr = take(sizeof(TickHeader));
-        uint8_t *reqs = take(sizeof(ReqDev) * kMaxTickRequests);
-        uint8_t *items = take(sizeof(Item) * kMaxTickItems);
         uint8_t *init = take(sizeof(int32_t) * kMaxTickRequests);
         uint8_t *fin = take(sizeof(int32_t) * kMaxTickRequests);
+        uint8_t *reqs = take(sizeof(ReqDev) * kMaxTickRequests + sizeof(Item) * (kMaxTickItems + 1));
+        uint8_t *items = reqs;
         uint8_t *rep = take(sizeof(Report) * kMaxTickRequests);
         if (d) {
             d->hdr = reinterpret_cast<TickHeader *>(hdr);
@@ -643,12 +861,12 @@ class Server {
     void build_candidates() {
         const int threads[2] = {256, 512};
         const int64_t items[2] = {32 << 10, 128 << 10};
-        const int smem[2] = {0, kSmemGroupsMax};
+        const int smem[2] = {0, kSmemGroupsAlways};
         for (int a : threads)
             for (int64_t b : items)
                 for (int c : smem) cands_.push_back(Cand{a, b, c});
         // Fixed shape (no tuning): 512 threads, 128 Ki-row items, shared memory
-        // aggregation up to the limit.
+        // aggregation of few groups always.
         best_ = (int)cands_.size() - 1;
         tuned_ = !opt_.autotune;
     }
@@ -685,7 +903,16 @@ class Server {
         }
     }
 
-    ReqDev req_dev(const Req &r, bool smem) const {
+    // Where `rows` rows of a request aggregate: in shared memory, by the first
+    // launch (0) or the second (1), or in device memory (-1).
+    static int smem_of(const Req &r, const Cand &c, int64_t rows) {
+        const int64_t ng = r.table->ngroups;
+        const bool pays = kSmemRowsPerGroup * ng <= std::min(rows, c.item_rows);
+        if (ng <= tick_smem_groups(c.threads) && (ng <= c.smem_groups || pays)) return 0;
+        return ng <= kMidGroups && pays ? 1 : -1;
+    }
+
+    ReqDev req_dev(const Req &r, const Cand &c, int smem) const {
         const ResidentTable &t = *r.table;
         const auto tv = t.join->table_dev();
         const size_t ng = (size_t)std::max<int64_t>(t.ngroups, 1);
@@ -704,7 +931,11 @@ class Server {
         d.out_sum = d.out_g + ng;
         d.out_cnt = d.out_g + 2 * ng;
         d.ngroups = (int32_t)t.ngroups;
-        d.use_smem = smem ? 1 : 0;
+        d.use_smem = smem >= 0 ? 1 : 0;
+        d.copies = 0;
+        const int64_t cap = smem > 0 ? kMidGroups : tick_smem_groups(c.threads);
+        while (d.copies < 5 && (t.ngroups << (d.copies + 1)) <= cap) d.copies++;
+        d.split = t.layout != kChains && r.rows < (1ll << 32) ? 1 : 0;
         return d;
     }
 
@@ -728,28 +959,44 @@ class Server {
         });
         int nreq = 0, nitems = 0, ninit = 0, nfinal = 0;
         int64_t budget = opt_.tick_rows, rows = 0;
+        items_[0].clear();
+        items_[1].clear();
+        // Items of about an eighth of a CTA's share of the tick, at least one
+        // step of the kernel.
+        int64_t due = 0;
+        for (const auto &r : order) due += r->rows - r->next_row;
+        due = std::min(due, budget);
+        const int64_t step = (int64_t)c.threads * kTickRowsPerThread;
+        const int64_t share = std::max(step, ceil_div(due, (int64_t)8 * rt_->sm_count * (1024 / c.threads)));
         Tick tick{s, tick_seq_, ci, 0, {}};
         std::vector<std::shared_ptr<Req>> keep;
         for (auto &r : order) {
             const int64_t left = r->rows - r->next_row;
             int64_t take = std::min(left, budget);
-            const int64_t item_rows = c.item_rows;
+            int64_t item_rows = std::min(c.item_rows, share);
+            const int smem = smem_of(*r, c, take);
+            // Groups in shared memory: an item's rows pay for their clearing and
+            // merging, and the second launch's CTAs get as many items each.
+            // Groups in device memory: an SM's atomics are the limit, so all SMs
+            // get some of the rows.
+            if (smem >= 0) item_rows = std::min(c.item_rows, std::max(item_rows, kSmemRowsPerGroup * r->table->ngroups));
+            else item_rows = std::min(item_rows, std::max(step, ceil_div(take, kMaxTickItems / 8)));
+            if (smem == 1) {
+                const int64_t turns = ceil_div(take, item_rows * rt_->sm_count);
+                item_rows = std::max((int64_t)kMidThreads * kTickRowsPerThread, ceil_div(take, turns * rt_->sm_count));
+            }
             const int64_t need_items = (take + item_rows - 1) / item_rows;
             if (nitems + need_items > kMaxTickItems) take = (int64_t)(kMaxTickItems - nitems) * item_rows;
             if (take <= 0 && left > 0) continue;
             const int idx = nreq++;
-            const bool smem = r->table->ngroups <= c.smem_groups;
-            hd.reqs[idx] = req_dev(*r, smem);
+            hd.reqs[idx] = req_dev(*r, c, smem);
             if (!r->inited) {
                 hd.init[ninit++] = idx;
                 r->inited = true;
             }
-            for (int64_t o = 0; o < take; o += item_rows) {
-                Item &it = hd.items[nitems++];
-                it.req = idx;
-                it.row0 = r->next_row + o;
-                it.rows = std::min(item_rows, take - o);
-            }
+            for (int64_t o = 0; o < take; o += item_rows)
+                items_[smem == 1].push_back(Item{idx, 0, r->next_row + o, std::min(item_rows, take - o)});
+            nitems = (int)(items_[0].size() + items_[1].size());
             r->next_row += take;
             budget -= take;
             rows += take;
@@ -761,25 +1008,27 @@ class Server {
         }
         if (nreq == 0) return;
         for (auto &r : tick.finals) active_.erase(std::find(active_.begin(), active_.end(), r));
-        hd.hdr->cursor = 0;
-        hd.hdr->n_items = nitems;
         hd.hdr->n_init = ninit;
         hd.hdr->n_final = nfinal;
+        // The items of the largest requests, last in the list, are taken first
+        // (the device takes them from its end): the end of a tick is short items.
+        int at = (int)ceil_div((int64_t)(sizeof(ReqDev) * nreq), (int64_t)sizeof(Item));
+        for (int q = 0; q < 2; q++) {
+            hd.hdr->cursor[q] = 0;
+            hd.hdr->n_items[q] = (int)items_[q].size();
+            hd.hdr->items_at[q] = at;
+            if (!items_[q].empty()) std::memcpy(hd.items + at, items_[q].data(), sizeof(Item) * items_[q].size());
+            at += (int)items_[q].size();
+        }
         tick.rows = rows;
         // Upload the used parts of the descriptors, then run the tick's graph.
         TickDev dd;
         layout(&dd, static_cast<uint8_t *>(sl.dev.get()));
-        auto up = [&](void *dst, const void *src, size_t bytes) {
-            if (bytes) KRV_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, rt_->stream));
-        };
-        up(dd.hdr, hd.hdr, sizeof(TickHeader));
-        up(dd.reqs, hd.reqs, sizeof(ReqDev) * nreq);
-        up(dd.items, hd.items, sizeof(Item) * nitems);
-        up(dd.init, hd.init, sizeof(int32_t) * ninit);
-        up(dd.final, hd.final, sizeof(int32_t) * nfinal);
+        const size_t used = (size_t)((uint8_t *)(hd.items + at) - (uint8_t *)hd.hdr);
+        KRV_CUDA(cudaMemcpyAsync(dd.hdr, hd.hdr, used, cudaMemcpyHostToDevice, rt_->stream));
         KRV_CUDA(cudaEventRecord(sl.start, rt_->stream));
-        KRV_CUDA(cudaGraphLaunch(graph_for(s, c.threads, dd, sl), rt_->stream));
-        rt_->launches += 3;
+        KRV_CUDA(cudaGraphLaunch(graph_for(s, c.threads, !items_[1].empty(), dd, sl), rt_->stream));
+        rt_->launches += items_[1].empty() ? 3 : 4;
         KRV_CUDA(cudaEventRecord(sl.done, rt_->stream));
         tick_seq_++;
         ticks_++;
@@ -787,27 +1036,28 @@ class Server {
         inflight_.push_back(std::move(tick));
     }
 
-    cudaGraphExec_t graph_for(int s, int threads, const TickDev &dd, Slot &sl) {
-        const int key = s * 4096 + threads;
+    cudaGraphExec_t graph_for(int s, int threads, bool mid, const TickDev &dd, Slot &sl) {
+        const int key = s * 4096 + threads * 2 + (mid ? 1 : 0);
         auto it = graphs_.find(key);
         if (it != graphs_.end()) return it->second;
         // The shape of the tick: the kernels read their counts from the
         // descriptors, so one graph serves every tick of this slot and shape.
         const int grid = rt_->sm_count * (threads == 256 ? 4 : 2);
-        const size_t smem = (size_t)kSmemGroupsMax * 24;
-        if (threads == 256)
-            KRV_CUDA(cudaFuncSetAttribute(tick_probe_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else
-            KRV_CUDA(cudaFuncSetAttribute(tick_probe_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const size_t smem = (size_t)tick_smem_groups(threads) * kSmemGroupBytes;
+        const size_t mid_smem = (size_t)kMidGroups * kSmemGroupBytes;
+        const auto probe = threads == 256 ? tick_probe_kernel<256, 0> : tick_probe_kernel<512, 0>;
+        const auto mid_probe = tick_probe_kernel<kMidThreads, 1>;
+        KRV_CUDA(cudaFuncSetAttribute(probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KRV_CUDA(cudaFuncSetAttribute(mid_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mid_smem));
         cudaStream_t cs;
         KRV_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            tick_init_kernel<<<rt_->sm_count * 2, 256, 0, cs>>>(dd);
-            if (threads == 256) tick_probe_kernel<256><<<grid, 256, smem, cs>>>(dd);
-            else tick_probe_kernel<512><<<grid, 512, smem, cs>>>(dd);
-            tick_final_kernel<<<rt_->sm_count * 2, 256, 0, cs>>>(dd);
+            tick_init_kernel<<<rt_->sm_count * 2, kChunkThreads, 0, cs>>>(dd);
+            if (mid) mid_probe<<<rt_->sm_count, kMidThreads, mid_smem, cs>>>(dd);
+            probe<<<grid, threads, smem, cs>>>(dd);
+            tick_final_kernel<<<rt_->sm_count * 2, kChunkThreads, 0, cs>>>(dd);
             cudaMemcpyAsync(sl.report_host, dd.report, sizeof(Report) * kMaxTickRequests, cudaMemcpyDeviceToHost, cs);
             e = cudaStreamEndCapture(cs, &graph);
         }
@@ -945,6 +1195,7 @@ class Server {
     std::map<int64_t, std::shared_ptr<Req>> reqs_;
     std::deque<std::shared_ptr<Req>> pending_, done_;
     std::vector<std::shared_ptr<Req>> active_;
+    std::vector<Item> items_[2];  // of the tick being formed, by launch
     std::deque<Tick> inflight_;
     int64_t next_table_ = 1, next_req_ = 1, tick_seq_ = 0;
     int64_t ticks_ = 0, requests_done_ = 0, rows_probed_ = 0, budget_used_ = 0;
