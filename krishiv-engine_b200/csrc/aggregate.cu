@@ -2882,7 +2882,8 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
         // when there is no such room) for as many as were counted.
         unsigned long long cold = (unsigned long long)ns;
         DBuf part_buf;
-        if ((uint64_t)ns * part_row_bytes_ <= kPartBufBytes) {
+        const uint64_t most = (uint64_t)ns * part_row_bytes_;
+        if (most <= kPartBufBytes && (rt_->budget == 0 || most <= (uint64_t)rt_->budget / 8)) {
             try {
                 part_buf = DBuf(rt_, (size_t)cold * part_row_bytes_);
             } catch (const Error &e) {

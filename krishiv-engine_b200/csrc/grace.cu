@@ -532,7 +532,7 @@ class GraceJoin {
                 counters_.build_keys += P.join->counters().build_keys;
                 counters_.table_slots += P.join->counters().table_slots;
             }
-        // A join over no build rows pads the NULL-key probe rows (left outer).
+        // A join over no build rows: the output's shape, and the fallback's padding.
         null_join_.reset(new HashJoin(rt_, spec_));
         null_join_->build_push(empty_like(build_types_));
         null_join_->build_finish();
@@ -1186,11 +1186,13 @@ class GraceJoin {
     void start(Prefetch &f, const std::vector<HostChunk> &hs, size_t &at) {
         std::vector<HostChunk> group;
         int64_t rows = 0;
-        while (at < hs.size() && (group.empty() || rows + hs[at].rows <= slice_rows())) {
-            rows += hs[at].rows;
-            group.push_back(hs[at++]);
+        size_t end = at;
+        while (end < hs.size() && (group.empty() || rows + hs[end].rows <= slice_rows())) {
+            rows += hs[end].rows;
+            group.push_back(hs[end++]);
         }
         start(f, group, probe_types_);
+        at = end;
     }
     void start(Prefetch &f, const std::vector<HostChunk> &group, const std::vector<DevCol> &types) {
         int64_t rows = 0;
