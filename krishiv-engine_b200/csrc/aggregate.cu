@@ -2615,9 +2615,31 @@ __global__ void __launch_bounds__(kPickThreads) hot_pick_kernel(AggPlanDev P, Ta
     __syncthreads();
     for (unsigned i = threadIdx.x; i < n; i += kPickThreads) atomicAdd(&s_bin[min(cnt[i], (unsigned)kPickBins - 1)], 1u);
     __syncthreads();
-    if (threadIdx.x == 0) {  // the lowest count that at most `most` keys reach
-        unsigned sum = 0, cut = kPickBins;
-        while (cut > 0 && sum + s_bin[cut - 1] <= (unsigned)most) sum += s_bin[--cut];
+    // The lowest count that at most `most` keys reach: every thread adds its
+    // bins up, a scan from the top says how many keys lie above them, and the
+    // thread whose bins pass `most` finds the place (one thread's walk down
+    // the bins took 30 us of the kernel's 35).
+    constexpr int kPer = kPickBins / kPickThreads;
+    static_assert(kPer * kPickThreads == kPickBins, "bins in whole shares");
+    __shared__ unsigned s_warp[kPickThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b0 = (kPickThreads - 1 - (int)threadIdx.x) * kPer;  // thread 0 has the highest counts
+    unsigned mine = 0;
+    for (int q = 0; q < kPer; q++) mine += s_bin[b0 + q];
+    unsigned incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned y = __shfl_up_sync(kFullMask, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    unsigned above = incl - mine;
+    for (int w = 0; w < warp; w++) above += s_warp[w];
+    const bool last = threadIdx.x == kPickThreads - 1;
+    if (above <= (unsigned)most && (above + mine > (unsigned)most || last)) {
+        unsigned sum = above, cut = (unsigned)(b0 + kPer);
+        while (cut > (unsigned)b0 && sum + s_bin[cut - 1] <= (unsigned)most) sum += s_bin[--cut];
         unsigned nb = 2;
         while (nb * 2 < sum) nb *= 2;
         s_cut = cut;
