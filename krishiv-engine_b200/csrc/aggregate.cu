@@ -2865,6 +2865,7 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
     const KeyIn key0 = key;
     for (int64_t row0 = 0; row0 < n; row0 += kPartSliceRows) {
         const int64_t ns = std::min<int64_t>(kPartSliceRows, n - row0);
+        index_pending();  // this slice looks the groups of the one before up
         SplitDev S{};
         S.hot_keys = part_hot_keys_.as<long long>();
         S.hot_gids = part_hot_gids_.as<uint32_t>();
