@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "krv_device.cuh"
+#include "limbs.h"
 #include "ops.h"
 
 namespace krv {
@@ -309,22 +310,16 @@ struct GroupSums {
 // one per lane, so that the lanes of a warp do not queue on one word.
 template <int CAP> struct SmemGroups {
     uint32_t *w;
-    // `many`: more than 2^32 rows may join (duplicate build keys): the count's
-    // carries go straight to device memory.
+    // `many`: more than 2^32 rows may join (duplicate build keys): what the
+    // count and the sum carry past their words goes straight to device memory,
+    // where such a request's sums have 128 bits.
     __device__ __forceinline__ void add(int g, int copies, int copy, bool many, const GroupSums &G, long long x) const {
         const int e = (g << copies) + copy;
         if (!many) atomicAdd(w + e, 1u);
         else if (atomicAdd(w + e, 1u) == 0xFFFFFFFFu) atomicAdd(G.cnt + g, 1ull << 32);
-        const uint32_t x0 = (uint32_t)x;
-        const uint32_t o0 = atomicAdd(w + CAP + e, x0);
-        const unsigned long long a1 = (unsigned long long)(uint32_t)(x >> 32) + (o0 + x0 < o0 ? 1u : 0u);
-        uint32_t a2 = (x < 0 ? 0xFFFFFFFFu : 0u) + (uint32_t)(a1 >> 32);
-        const uint32_t x1 = (uint32_t)a1;
-        if (x1) {
-            const uint32_t o1 = atomicAdd(w + 2 * CAP + e, x1);
-            a2 += o1 + x1 < o1 ? 1u : 0u;
-        }
-        if (a2) atomicAdd(w + 3 * CAP + e, a2);
+        uint32_t *sum = w + CAP + e;
+        const int over = sum96_add([=](int p, uint32_t v) { return atomicAdd(sum + p * CAP, v); }, x);
+        if (many && over) atomicAdd(G.hi + g, (unsigned long long)((long long)over * (1ll << 32)));
     }
     __device__ __forceinline__ void clear(const ReqDev &R, int threads) const {
         const int n = R.ngroups << R.copies;
