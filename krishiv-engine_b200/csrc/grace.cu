@@ -527,7 +527,7 @@ class GraceJoin {
         DeviceGuard g(rt_);
         if (!schema_) fail(KRV_INVALID_ARGUMENT, "a partitioned join needs the build side's schema: push a build batch");
         for (auto &P : parts_)
-            if (!P.spilled) {
+            if (!P.spilled && !P.join->built()) {  // built: by a call that then failed
                 P.join->build_finish();
                 counters_.build_keys += P.join->counters().build_keys;
                 counters_.table_slots += P.join->counters().table_slots;

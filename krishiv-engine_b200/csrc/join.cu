@@ -1397,7 +1397,6 @@ HashJoin::TableDev HashJoin::table_dev() const {
 void HashJoin::build_finish() {
     if (built_) fail(KRV_INVALID_ARGUMENT, "build_finish called twice");
     DeviceGuard g(rt_);
-    built_ = true;
     arena_.rows = build_rows_;
     arena_.cols.clear();
     for (size_t i = 0; i < arena_cols_.size(); i++) {
@@ -1482,6 +1481,7 @@ void HashJoin::build_finish() {
             filter_ = build_key_filter(rt_, o, key, spec_.null_safe[0] ? nullptr : &ks);
         }
     }
+    built_ = true;  // only now: a call that failed (for memory, say) may be made again
 }
 
 static std::vector<int> projection(int n, const int32_t *cols, int ncols) {
