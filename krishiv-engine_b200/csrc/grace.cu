@@ -647,11 +647,13 @@ class GraceJoin {
         }
         for (int pc : pcols) o.cols.push_back(in.cols[pc]);
         if (!bcols.empty() && (!null_data_ || in.rows > null_rows_)) {
+            auto data = std::make_shared<DBuf>(rt_, (size_t)in.rows * 8);
+            auto valid = std::make_shared<DBuf>(rt_, (size_t)ceil_div(in.rows, 32) * 4 + 8);
+            KRV_CUDA(cudaMemsetAsync(data->get(), 0, data->bytes(), rt_->stream));
+            KRV_CUDA(cudaMemsetAsync(valid->get(), 0, valid->bytes(), rt_->stream));
+            null_data_ = data;
+            null_valid_ = valid;
             null_rows_ = in.rows;
-            null_data_ = std::make_shared<DBuf>(rt_, (size_t)null_rows_ * 8);
-            null_valid_ = std::make_shared<DBuf>(rt_, (size_t)ceil_div(null_rows_, 32) * 4 + 8);
-            KRV_CUDA(cudaMemsetAsync(null_data_->get(), 0, null_data_->bytes(), rt_->stream));
-            KRV_CUDA(cudaMemsetAsync(null_valid_->get(), 0, null_valid_->bytes(), rt_->stream));
         }
         for (int bc : bcols) {
             DevCol c;
@@ -813,14 +815,19 @@ class GraceJoin {
         }
         // Ruled-out rows that did not fit their call's output, padded now, then
         // the deferred rows of resident partitions, by their resident tables.
-        // The next group crosses the host link while this one is joined.
-        while (later_.pending || start_later()) {
-            const int p = later_part_;
-            DevBatch pb = take(later_);
-            start_later();
-            DevBatch o = p < 0 ? padded(std::move(pb), 0) : parts_[p].join->probe(pb);
-            if (later_part_ != p || !later_.pending)
-                for (int q = 0; q < (later_.pending ? later_part_ : nparts_); q++) parts_[q].join.reset();  // done
+        // The next group crosses the host link while this one is joined. A
+        // group taken stays a member until its output is there, and a task
+        // listed until its table is built: after a call that fails for memory
+        // the next one goes on with the same rows.
+        while (taken_.live || later_.pending || start_later()) {
+            if (!taken_.live) taken_ = Taken{take(later_), later_part_, true};
+            if (!later_.pending) ahead([&] { start_later(); });
+            const int p = taken_.part;
+            DevBatch o = needed([&] { return p < 0 ? padded(taken_.batch, 0) : parts_[p].join->probe(taken_.batch); });
+            taken_ = Taken{};
+            // the tables before the next group's are done
+            const int next = later_.pending ? later_part_ : pad_chunk_ < pad_later_.size() ? 0 : deferred_part_;
+            for (int q = 0; q < next; q++) parts_[q].join.reset();
             counters_.output_rows += o.rows;
             if (o.rows > 0) {
                 out = o;
@@ -834,13 +841,18 @@ class GraceJoin {
                 continue;
             }
             if (cur_join_) {
-                if (prefetch_.pending || cur_probe_ < cur_.probe_host.size()) {
-                    if (!prefetch_.pending) start(prefetch_, cur_.probe_host, cur_probe_);
-                    DevBatch pb = take(prefetch_);
+                if (probing_.live || prefetch_.pending || cur_probe_ < cur_.probe_host.size()) {
+                    if (!probing_.live) {
+                        if (!prefetch_.pending) start(prefetch_, cur_.probe_host, cur_probe_);
+                        probing_ = Taken{take(prefetch_), 0, true};
+                    }
                     // the next group crosses the host link while this one is probed
-                    if (cur_probe_ < cur_.probe_host.size()) start(prefetch_, cur_.probe_host, cur_probe_);
-                    else start_next_build();
-                    DevBatch o = cur_join_->probe(pb);
+                    ahead([&] {
+                        if (!prefetch_.pending && cur_probe_ < cur_.probe_host.size()) start(prefetch_, cur_.probe_host, cur_probe_);
+                        else if (!prefetch_.pending) start_next_build();
+                    });
+                    DevBatch o = needed([&] { return cur_join_->probe(probing_.batch); });
+                    probing_ = Taken{};
                     counters_.output_rows += o.rows;
                     if (o.rows == 0) continue;
                     out = o;
@@ -850,39 +862,49 @@ class GraceJoin {
                 cur_ = Task{};
             }
             if (tasks_.empty()) return false;
-            Task t = std::move(tasks_.front());
-            tasks_.pop_front();
+            Task &t = tasks_.front();
             int64_t rows = 0;
             for (const HostChunk &c : t.build_host) rows += c.rows;
-            if (t.probe_host.empty()) continue;  // no probe rows: nothing to emit
+            if (t.probe_host.empty()) {  // no probe rows: nothing to emit
+                tasks_.pop_front();
+                continue;
+            }
             if (est_part_bytes(rows) > resident_cap() && t.level < kMaxLevel && !no_shrink(t, rows)) {
-                split(t);
+                split_front();
                 continue;
             }
             if (est_part_bytes(rows) > resident_cap()) {
                 // Splitting cannot shrink it (one heavy key): the fallback.
-                start_fallback(std::move(t));
+                start_fallback();
                 continue;
             }
             krv_join_spec js = spec_;
             js.build_rows_hint = rows;
-            cur_join_.reset(new HashJoin(rt_, js));
-            if (rows && !next_build_.pending) start(next_build_, t.build_host, build_types_);
+            std::unique_ptr<HashJoin> join;
+            if (!prefetch_.pending) cur_probe_ = 0;
+            bool early = true;  // not when the table's memory went to them
+            needed([&] {
+                join.reset(new HashJoin(rt_, js));
+                if (rows && !next_build_.pending) start(next_build_, t.build_host, build_types_);
+                // the first probe rows cross the host link while the table is built
+                if (early && !prefetch_.pending) ahead([&] { start(prefetch_, t.probe_host, cur_probe_); });
+                early = false;
+                if (rows == 0) join->build_push(empty_like(build_types_));
+                else join->build_adopt(take(next_build_));
+                join->build_finish();
+                return DevBatch{};
+            });
+            cur_join_ = std::move(join);
             cur_ = std::move(t);
+            tasks_.pop_front();
             cur_rows_ = rows;
-            cur_probe_ = 0;
-            // the first probe rows cross the host link while the table is built
-            start(prefetch_, cur_.probe_host, cur_probe_);
-            if (rows == 0) cur_join_->build_push(empty_like(build_types_));
-            else cur_join_->build_adopt(take(next_build_));
-            cur_join_->build_finish();
             counters_.build_keys += cur_join_->counters().build_keys;
             counters_.table_slots += cur_join_->counters().table_slots;
         }
     }
 
     bool done() const {
-        return finishing_ && !later_.pending && pad_chunk_ >= pad_later_.size() && deferred_part_ >= nparts_ &&
+        return finishing_ && !taken_.live && !later_.pending && pad_chunk_ >= pad_later_.size() && deferred_part_ >= nparts_ &&
                !cur_join_ && tasks_.empty() && !fb_.active;
     }
     // A zero-row batch of the output's shape.
@@ -1124,6 +1146,8 @@ class GraceJoin {
     std::vector<HostChunk> spill(const Rows &s, const std::vector<DevCol> &types) {
         std::vector<HostChunk> h(s.runs.size());
         if (s.rows == 0) return h;
+        std::vector<uint8_t *> host;  // all of it first: no copy is under way when there is none
+        for (const DevCol &t : types) host.push_back(host_alloc((size_t)s.rows * t.type.width()));
         cudaEvent_t ready;
         KRV_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
         KRV_CUDA(cudaEventRecord(ready, rt_->stream));
@@ -1132,7 +1156,7 @@ class GraceJoin {
         InFlight f;
         for (size_t c = 0; c < types.size(); c++) {
             const size_t w = (size_t)types[c].type.width(), bytes = (size_t)s.rows * w;
-            uint8_t *p = host_alloc(bytes);
+            uint8_t *p = host[c];
             KRV_CUDA(cudaMemcpyAsync(p, s.cols[c]->get(), bytes, cudaMemcpyDeviceToHost, cs_));
             for (size_t i = 0; i < s.runs.size(); i++) {
                 h[i].rows = s.runs[i].second;
@@ -1182,6 +1206,7 @@ class GraceJoin {
         DBuf table;
         cudaEvent_t ready = nullptr;
         bool pending = false;
+        size_t from = 0;  // of the probe chunks: its first one
     };
     void start(Prefetch &f, const std::vector<HostChunk> &hs, size_t &at) {
         std::vector<HostChunk> group;
@@ -1192,22 +1217,58 @@ class GraceJoin {
             group.push_back(hs[end++]);
         }
         start(f, group, probe_types_);
+        f.from = at;
         at = end;
     }
     void start(Prefetch &f, const std::vector<HostChunk> &group, const std::vector<DevCol> &types) {
         int64_t rows = 0;
         for (const HostChunk &h : group) rows += h.rows;
-        f.batch = alloc_like(types, rows);  // allocated in the join's stream order
-        f.table = DBuf(rt_, group.size() * f.batch.cols.size() * sizeof(GatherRun));
+        DevBatch batch = alloc_like(types, rows);  // allocated in the join's stream order
+        DBuf table(rt_, group.size() * batch.cols.size() * sizeof(GatherRun));
+        if (!f.ready) KRV_CUDA(cudaEventCreateWithFlags(&f.ready, cudaEventDisableTiming));
         cudaEvent_t ready;
         KRV_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
         KRV_CUDA(cudaEventRecord(ready, rt_->stream));
         KRV_CUDA(cudaStreamWaitEvent(cs_, ready, 0));
         KRV_CUDA(cudaEventDestroy(ready));
-        copy_in(group, f.batch, f.table, cs_);
-        if (!f.ready) KRV_CUDA(cudaEventCreateWithFlags(&f.ready, cudaEventDisableTiming));
-        KRV_CUDA(cudaEventRecord(f.ready, cs_));
+        f.batch = std::move(batch);
+        f.table = std::move(table);
         f.pending = true;
+        copy_in(group, f.batch, f.table, cs_);
+        KRV_CUDA(cudaEventRecord(f.ready, cs_));
+    }
+    // Loads rows that are not needed yet; without memory for them they wait
+    // in host memory until they are.
+    template <class F> void ahead(F f) {
+        try {
+            f();
+        } catch (const Error &e) {
+            if (e.code != KRV_NEED_MEMORY) throw;
+        }
+    }
+    // The same call's own work: when its memory is held by rows loaded ahead,
+    // those are given up (they are still in host memory) and it runs again.
+    template <class F> DevBatch needed(F f) {
+        try {
+            return f();
+        } catch (const Error &e) {
+            if (e.code != KRV_NEED_MEMORY || !give_up_ahead()) throw;
+        }
+        return f();
+    }
+    bool give_up_ahead() {
+        const bool any = later_.pending || prefetch_.pending || next_build_.pending;
+        if (later_.pending) {
+            take(later_);
+            if (later_part_ < 0) pad_chunk_ = later_.from;
+            else deferred_part_ = later_part_, deferred_chunk_ = later_.from;
+        }
+        if (prefetch_.pending) {
+            take(prefetch_);
+            cur_probe_ = prefetch_.from;
+        }
+        if (next_build_.pending) take(next_build_);
+        return any;
     }
     DevBatch take(Prefetch &f) {
         KRV_CUDA(cudaStreamWaitEvent(rt_->stream, f.ready, 0));
@@ -1337,9 +1398,18 @@ class GraceJoin {
         return true;
     }
 
-    void start_fallback(Task t) {
+    void start_fallback() {
+        Task &t = tasks_.front();
+        DBuf matched;
+        if (spec_.join_type == KRV_JOIN_LEFT_OUTER) {
+            int64_t rows = 0;
+            for (const HostChunk &c : t.probe_host) rows += c.rows;
+            matched = DBuf(rt_, (size_t)std::max<int64_t>(rows, 1));
+            KRV_CUDA(cudaMemsetAsync(matched.get(), 0, matched.bytes(), rt_->stream));
+        }
         fallbacks_++;
         fb_ = Fallback{};
+        fb_.matched = std::move(matched);
         fb_.active = true;
         std::vector<HostChunk> g;
         int64_t grows = 0;
@@ -1359,10 +1429,7 @@ class GraceJoin {
             base += c.rows;
         }
         fb_.probe_host = std::move(t.probe_host);
-        if (spec_.join_type == KRV_JOIN_LEFT_OUTER) {
-            fb_.matched = DBuf(rt_, (size_t)std::max<long long>(base, 1));
-            KRV_CUDA(cudaMemsetAsync(fb_.matched.get(), 0, fb_.matched.bytes(), rt_->stream));
-        }
+        tasks_.pop_front();
     }
 
     // The probe chunk at `at` with its row ids as a last column.
@@ -1410,9 +1477,10 @@ class GraceJoin {
                 int64_t rows = 0;
                 for (const HostChunk &c : fb_.groups[fb_.group]) rows += c.rows;
                 js.build_rows_hint = rows;
-                fb_.join.reset(new HashJoin(rt_, js));
-                fb_.join->build_adopt(load_all(fb_.groups[fb_.group], build_types_));
-                fb_.join->build_finish();
+                std::unique_ptr<HashJoin> join(new HashJoin(rt_, js));
+                join->build_adopt(load_all(fb_.groups[fb_.group], build_types_));
+                join->build_finish();
+                fb_.join = std::move(join);
                 fb_.probe_at = 0;
             }
             if (fb_.probe_at == fb_.probe_host.size()) {
@@ -1420,8 +1488,8 @@ class GraceJoin {
                 fb_.group++;
                 return false;
             }
-            const size_t at = fb_.probe_at++;
-            DevBatch o = fb_.join->probe(load_with_ids(at));
+            DevBatch o = fb_.join->probe(load_with_ids(fb_.probe_at));
+            fb_.probe_at++;
             // the id column follows the probe columns
             const int idc = spec_.n_probe_out < 0 ? (int)probe_types_.size() : spec_.n_probe_out;
             if (fb_.matched.get() && o.rows) {
@@ -1441,7 +1509,7 @@ class GraceJoin {
             fb_ = Fallback{};
             return false;
         }
-        const size_t at = fb_.probe_at++;
+        const size_t at = fb_.probe_at;
         DevBatch b = load(fb_.probe_host[at], probe_types_);
         DevBatch keep = alloc_like(probe_types_, b.rows);
         PartArgs A{};
@@ -1458,11 +1526,10 @@ class GraceJoin {
         }
         keep.rows = (int64_t)read_scalar<unsigned long long>(rt_, cnt.get());
         for (DevCol &c : keep.cols) c.length = keep.rows;
-        if (keep.rows == 0) return false;
-        DevBatch o = null_join_->probe(keep);
-        counters_.output_rows += o.rows;
-        out = o;
-        return true;
+        if (keep.rows) out = null_join_->probe(keep);
+        fb_.probe_at++;
+        counters_.output_rows += keep.rows;
+        return keep.rows > 0;
     }
 
     void split_side(const std::vector<HostChunk> &from, const std::vector<DevCol> &types, int key, int level,
@@ -1480,14 +1547,15 @@ class GraceJoin {
         }
     }
 
-    // Splits task `t` 8 ways with the next level of hash bits, chunk by chunk.
-    void split(Task &t) {
-        const int level = t.level + 1;
+    // Splits the first task 8 ways with the next level of hash bits, chunk by chunk.
+    void split_front() {
+        const Task &t = tasks_.front();
         std::vector<Task> sub(8);
-        for (auto &s : sub) s.level = level;
-        split_side(t.build_host, build_types_, spec_.build_keys[0], level, sub, &Task::build_host);
-        split_side(t.probe_host, probe_types_, spec_.probe_keys[0], level, sub, &Task::probe_host);
+        for (auto &s : sub) s.level = t.level + 1;
+        split_side(t.build_host, build_types_, spec_.build_keys[0], t.level + 1, sub, &Task::build_host);
+        split_side(t.probe_host, probe_types_, spec_.probe_keys[0], t.level + 1, sub, &Task::probe_host);
         splits_ += 8;
+        tasks_.pop_front();
         for (auto &s : sub) tasks_.push_front(std::move(s));
     }
 
@@ -1527,6 +1595,12 @@ class GraceJoin {
     size_t inflight_bytes_ = 0;
     Prefetch prefetch_, later_, next_build_;
     int later_part_ = -1;
+    // The group of rows being joined: of later_ (part: its later_part_), of prefetch_.
+    struct Taken {
+        DevBatch batch;
+        int part = 0;
+        bool live = false;
+    } taken_, probing_;
     // The NULL build columns of padded rows
     std::shared_ptr<DBuf> null_data_, null_valid_;
     int64_t null_rows_ = 0;
