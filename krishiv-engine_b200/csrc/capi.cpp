@@ -98,6 +98,19 @@ DevBatch pop(std::vector<DevBatch> &pending) {
     return b;
 }
 
+// Exports `b`; one that had waited in `pending` waits on when that fails (a
+// slice's bitmaps may need memory to be aligned).
+template <bool Device, class Out>
+void hand_out(krv::Runtime *rt, DevBatch &b, std::vector<DevBatch> &pending, bool waited, Out *out, ArrowSchema *out_schema) {
+    try {
+        if constexpr (Device) krv::export_device(rt, b, out, out_schema);
+        else krv::export_host(rt, b, out, out_schema);
+    } catch (...) {
+        if (waited) pending.push_back(std::move(b));
+        throw;
+    }
+}
+
 // The first piece of several output batches; the rest wait in `pending`.
 DevBatch take_all(std::vector<DevBatch> bs, int64_t max_rows, std::vector<DevBatch> &pending) {
     std::vector<DevBatch> pieces;
@@ -279,6 +292,7 @@ static krv_status join_probe_impl(krv_join *j, const In *in, const ArrowSchema *
         krv::Runtime *rt = &j->owner->rt;
         krv::DeviceGuard g(rt);
         DevBatch b;
+        const bool waited = !in;
         if (in) {
             if (!j->pending.empty()) krv::fail(KRV_INVALID_ARGUMENT, "drain pending output (input NULL) first");
             DevBatch inb;
@@ -302,8 +316,7 @@ static krv_status join_probe_impl(krv_join *j, const In *in, const ArrowSchema *
             if (j->pending.empty()) krv::fail(KRV_INVALID_ARGUMENT, "no pending output and no input");
             b = pop(j->pending);
         }
-        if constexpr (Device) krv::export_device(rt, b, out, out_schema);
-        else krv::export_host(rt, b, out, out_schema);
+        hand_out<Device>(rt, b, j->pending, waited, out, out_schema);
         return j->pending.empty() ? KRV_NEED_MORE_INPUT : KRV_HAVE_MORE_OUTPUT;
     });
 }
@@ -325,7 +338,8 @@ static krv_status join_finish_impl(krv_join *j, Out *out, ArrowSchema *out_schem
         krv::Runtime *rt = &j->owner->rt;
         krv::DeviceGuard g(rt);
         DevBatch b;
-        if (!j->pending.empty()) {
+        const bool waited = !j->pending.empty();
+        if (waited) {
             b = pop(j->pending);
         } else if (j->g) {
             DevBatch next;
@@ -334,8 +348,7 @@ static krv_status join_finish_impl(krv_join *j, Out *out, ArrowSchema *out_schem
         } else {
             b = take_first(j->j->finish(), j->j->spec().max_output_rows, j->pending);
         }
-        if constexpr (Device) krv::export_device(rt, b, out, out_schema);
-        else krv::export_host(rt, b, out, out_schema);
+        hand_out<Device>(rt, b, j->pending, waited, out, out_schema);
         const bool more = !j->pending.empty() || (j->g && !krv::grace_done(j->g));
         return more ? KRV_HAVE_MORE_OUTPUT : KRV_FINISHED;
     });
@@ -451,19 +464,17 @@ static krv_status agg_output_impl(krv_agg *a, Out *out, ArrowSchema *out_schema)
         krv::Runtime *rt = &a->owner->rt;
         krv::DeviceGuard g(rt);
         DevBatch b;
+        const bool waited = a->produced;
         if (!a->produced) {
-            a->produced = true;
-            krv_agg_spec spec{};
-            (void)spec;
             DevBatch all = krv::agg_result(a->a);
+            a->produced = true;
             b = take_first(std::move(all), 0, a->pending);
         } else if (!a->pending.empty()) {
             b = pop(a->pending);
         } else {
             krv::fail(KRV_INVALID_ARGUMENT, "the aggregate's output was already returned");
         }
-        if constexpr (Device) krv::export_device(rt, b, out, out_schema);
-        else krv::export_host(rt, b, out, out_schema);
+        hand_out<Device>(rt, b, a->pending, waited, out, out_schema);
         return a->pending.empty() ? KRV_FINISHED : KRV_HAVE_MORE_OUTPUT;
     });
 }

@@ -528,7 +528,7 @@ static std::shared_ptr<DBuf> aligned_validity(Runtime *rt, const DevCol &c) {
 
 void export_host(Runtime *rt, const DevBatch &b, ArrowArray *out, ArrowSchema *out_schema) {
     const size_t n = b.cols.size();
-    auto *p = new HostArrayPriv();
+    auto p = std::make_unique<HostArrayPriv>();
     p->bufs.reserve(2 * n);
     p->child_bufs.resize(n);
     p->child_storage.resize(n);
@@ -587,13 +587,13 @@ void export_host(Runtime *rt, const DevBatch &b, ArrowArray *out, ArrowSchema *o
     out->n_children = (int64_t)n;
     out->children = n ? p->children.data() : nullptr;
     out->release = release_host_array;
-    out->private_data = p;
+    out->private_data = p.release();
     if (out_schema) export_schema(b, out_schema);
 }
 
 void export_device(Runtime *rt, const DevBatch &b, ArrowDeviceArray *out, ArrowSchema *out_schema) {
     const size_t n = b.cols.size();
-    auto *p = new DevArrayPriv();
+    auto p = std::make_unique<DevArrayPriv>();
     p->child_bufs.resize(n);
     p->child_storage.resize(n);
     p->children.resize(n);
@@ -624,7 +624,7 @@ void export_device(Runtime *rt, const DevBatch &b, ArrowDeviceArray *out, ArrowS
     out->array.n_children = (int64_t)n;
     out->array.children = n ? p->children.data() : nullptr;
     out->array.release = release_dev_array;
-    out->array.private_data = p;
+    out->array.private_data = p.release();
     out->device_id = rt->device;
     out->device_type = ARROW_DEVICE_CUDA;
     out->sync_event = nullptr;

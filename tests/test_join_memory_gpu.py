@@ -1,5 +1,7 @@
 """Joins when the runtime's budget runs out: a call that fails for memory may be
 made again, and what it was called on is as it was before. Exact."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -56,4 +58,41 @@ def test_build_finish_may_be_called_again(kb, small, partitioned):
     key, v = (np.concatenate([g[i] for g in got]) for i in range(2))
     assert len(key) == n and np.array_equal(np.sort(v), np.arange(n)) and np.array_equal(k[v], key)
     assert j.counters()["build_keys"] == n
+    j.close()
+
+
+@pytest.mark.parametrize("call", ["probe", "finish"])
+def test_a_slice_that_cannot_be_handed_out_waits(kb, small, call):
+    n = 1_000_003  # in slices whose bitmaps take more than ballast leaves
+    k = np.arange(n)
+    # probe: unmatched rows padded; finish: the full outer join's build rows that no row matched
+    j = kb.HashJoin(small, kb.join_spec("full_outer", probe_out=[0], build_out=[1], max_output_rows=196_608))
+    build, probe = (k + n, k[:10]) if call == "finish" else (k[:10] + n, k)
+    j.build_push_device(kb.DeviceBatch([column("k", build), column("v", build * 3)]))
+    j.build_finish()
+    rows = []
+
+    def take(call_again):
+        arr, sch = kb.ArrowDeviceArray(), kb.ArrowSchema()
+        st = call_again(C.byref(arr), C.byref(sch))
+        if st != kb.NEED_MEMORY:
+            r = kb.DeviceResult(arr, sch)
+            null = np.unpackbits(r.valid[1 if call == "probe" else 0].cpu().numpy(), bitorder="little")[:r.rows] == 0
+            rows.extend((r.columns[0] if call == "probe" else r.columns[1]).cpu().numpy()[null].tolist())
+        return kb.check(st) if st != kb.NEED_MEMORY else st
+
+    p, lib = kb.DeviceBatch([column("k", probe)]), kb.lib()
+    st = take(lambda a, s: lib.krv_join_probe_device(j.h, C.byref(p.dev), C.byref(p.schema), a, s))
+    failed = 0
+    more = lambda a, s: (lib.krv_join_probe_device(j.h, None, None, a, s) if call == "probe"  # noqa: E731
+                         else lib.krv_join_finish_device(j.h, a, s))
+    if call == "finish":
+        rows.clear()
+        st = take(more)
+    while st == kb.HAVE_MORE_OUTPUT:
+        b = ballast(kb, small, BUDGET, 0)
+        failed += take(more) == kb.NEED_MEMORY
+        b.close()
+        st = take(more)
+    assert failed >= 3 and sorted(rows) == (k.tolist() if call == "probe" else (build * 3).tolist())
     j.close()
