@@ -303,14 +303,20 @@ static krv_status join_probe_impl(krv_join *j, const In *in, const ArrowSchema *
                 hb.reset(new krv::HostBorrow(rt));
                 inb = krv::import_host(rt, in, in_schema, krv::HostRead::Copy, krv::Var::Allow);
             }
-            if (j->g) {
-                std::vector<DevBatch> outs = krv::grace_probe(j->g, inb);
-                if (outs.empty()) outs.push_back(krv::grace_empty_output(j->g));
-                b = take_all(std::move(outs), j->spec().max_output_rows, j->pending);
-            } else {
-                b = take_first(j->j->probe(inb), j->j->spec().max_output_rows, j->pending);
-                // the caller's device buffers are its own again when the call returns
-                if (Device && j->j->emitting()) KRV_CUDA(cudaStreamSynchronize(rt->stream));
+            // the caller's device buffers are its own again when the call
+            // returns, and when it fails
+            try {
+                if (j->g) {
+                    std::vector<DevBatch> outs = krv::grace_probe(j->g, inb);
+                    if (outs.empty()) outs.push_back(krv::grace_empty_output(j->g));
+                    b = take_all(std::move(outs), j->spec().max_output_rows, j->pending);
+                } else {
+                    b = take_first(j->j->probe(inb), j->j->spec().max_output_rows, j->pending);
+                    if (Device && j->j->emitting()) KRV_CUDA(cudaStreamSynchronize(rt->stream));
+                }
+            } catch (...) {
+                if (Device) cudaStreamSynchronize(rt->stream);
+                throw;
             }
         } else {
             if (j->pending.empty()) krv::fail(KRV_INVALID_ARGUMENT, "no pending output and no input");

@@ -1505,7 +1505,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     const DevBatch &in = coded_ ? coded_in : outer_in;
     const int jt = spec_.join_type;
     const int64_t n = in.rows;
-    emitting_ = false;
+    emitting_ = n > 0;  // from here on kernels that read the batch are queued, until total() has waited
     counters_.probe_rows += n;
     if (probe_types_.empty()) {
         for (const DevCol &c : in.cols) {
@@ -1698,6 +1698,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     auto total = [&]() -> int64_t {  // waits for the scan
         if (none) return 0;
         KRV_CUDA(cudaStreamSynchronize(rt_->stream));
+        emitting_ = false;
         volatile unsigned long long *seen =
             reinterpret_cast<volatile unsigned long long *>(static_cast<uint8_t *>(rt_->status_host) + 64);
         if (seen[1] & ST_TOO_MANY)
@@ -1757,6 +1758,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
             E.tiles = tiles.as<unsigned long long>() + row0 / kTileRows;
             E.next = next_.as<uint32_t>();
             E.pad = pads && pairs;
+            emitting_ = true;
             launch_emit(how, E, od);
         }
     };
@@ -1782,12 +1784,12 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     for (DevCol &c : out.cols) c.length = m;
     for (const VarOut &v : vars) {
         const DevCol meta = out.cols[v.pos];
+        emitting_ = emitting_ || (v.side == 0 && m > 0);
         out.cols[v.pos] = var_gather(rt_, var_src(v.side, v.col, &in), idx[v.side].as<long long>(), m, meta.type,
                                      meta.nullable, meta.name);
     }
     counters_.output_rows += m;
     remember_shape(out);
-    emitting_ = how == kChains && m > 0;
     return out;
 }
 
