@@ -574,15 +574,14 @@ class GraceJoin {
     // that goes to host memory like the rows of spilled partitions (and is
     // joined at finish by the same resident tables). Padded rows come first,
     // those of the slices yet to come too: they are the partition pass's own
-    // copy of the probe columns beside shared NULL columns, so of the same
-    // bytes of output they keep twice as many rows off the host link.
+    // copy of the probe columns beside NULL columns, so they cost no join.
     void probe_slice(const DevBatch &in, std::vector<DevBatch> &out, Share &share) {
         const bool left = spec_.join_type == KRV_JOIN_LEFT_OUTER;
         Counted k = count(in, spec_.probe_keys[0], 0, parts_bits_, left, bloom_ ? kFilterTest : kFilterNone);
         const int64_t nulls = left ? (int64_t)k.rows[nparts_] : 0;
         const int64_t ruled_out = left ? (int64_t)k.rows[nparts_ + 1] : 0;
         counters_filtered_ += (int64_t)k.rows[nparts_ + 1];  // counted whether the rows are kept or dropped
-        const int64_t out_cap = budget_ / 8, pad_bytes = probe_row_bytes();
+        const int64_t out_cap = budget_ / 8, pad_bytes = padded_row_bytes();
         share.rows += in.rows;
         share.rows_left -= in.rows;
         share.ruled_out += ruled_out;
@@ -630,7 +629,8 @@ class GraceJoin {
 
     // The output rows of probe rows without a match (owned columns), the
     // first `nulls` of them with a NULL key: their columns as they are, the
-    // build columns NULL (one zeroed buffer that all of them share).
+    // build columns NULL. Every column has memory of its own: the caller may
+    // write to it.
     DevBatch padded(DevBatch in, int64_t nulls) {
         DevBatch o;
         o.rows = in.rows;
@@ -646,25 +646,10 @@ class GraceJoin {
             k.valid_off = 0;
         }
         for (int pc : pcols) o.cols.push_back(in.cols[pc]);
-        if (!bcols.empty() && (!null_data_ || in.rows > null_rows_)) {
-            auto data = std::make_shared<DBuf>(rt_, (size_t)in.rows * 8);
-            auto valid = std::make_shared<DBuf>(rt_, (size_t)ceil_div(in.rows, 32) * 4 + 8);
-            KRV_CUDA(cudaMemsetAsync(data->get(), 0, data->bytes(), rt_->stream));
-            KRV_CUDA(cudaMemsetAsync(valid->get(), 0, valid->bytes(), rt_->stream));
-            null_data_ = data;
-            null_valid_ = valid;
-            null_rows_ = in.rows;
-        }
         for (int bc : bcols) {
-            DevCol c;
-            c.type = build_types_[bc].type;
-            c.name = build_types_[bc].name;
-            c.nullable = true;
-            c.length = in.rows;
-            c.hold_data = null_data_;
-            c.data = null_data_->get();
-            c.hold_valid = null_valid_;
-            c.valid = null_valid_->as<uint8_t>();
+            DevCol c = make_col(rt_, build_types_[bc].type, in.rows, true, build_types_[bc].name);
+            KRV_CUDA(cudaMemsetAsync(c.hold_data->get(), 0, c.hold_data->bytes(), rt_->stream));
+            KRV_CUDA(cudaMemsetAsync(c.hold_valid->get(), 0, c.hold_valid->bytes(), rt_->stream));
             o.cols.push_back(c);
         }
         return o;
@@ -781,9 +766,11 @@ class GraceJoin {
         return std::max<int64_t>(b, 8);
     }
 
-    int64_t probe_row_bytes() const {
+    // Bytes of one padded row: the partitioned copy of the probe columns, the NULL columns.
+    int64_t padded_row_bytes() const {
         int64_t b = 0;
         for (const DevCol &c : probe_types_) b += c.type.width();
+        for (int bc : projection(spec_.n_build_out, spec_.build_out, (int)build_types_.size())) b += build_types_[bc].type.width();
         return b;
     }
 
@@ -1601,9 +1588,6 @@ class GraceJoin {
         int part = 0;
         bool live = false;
     } taken_, probing_;
-    // The NULL build columns of padded rows
-    std::shared_ptr<DBuf> null_data_, null_valid_;
-    int64_t null_rows_ = 0;
     uint8_t *cur_block_ = nullptr;
     size_t cur_block_used_ = 0;
     krv_join_counters counters_{};
