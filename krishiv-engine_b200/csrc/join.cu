@@ -374,10 +374,11 @@ __device__ __forceinline__ void emit_round(const OutDev &out, bool want, unsigne
 //     every tile of kTileRows rows; tile_scan_kernel turns the sums into every
 //     tile's first output row and tells the host the total;
 //  2. emit_kernel, into output columns of exactly that size, stages each
-//     tile's (probe row, build row) pairs in shared memory in output order,
-//     kWindow at a time, and writes them column by column: neighbouring
-//     threads write neighbouring output rows, so stores are coalesced, and a
-//     warp owns whole validity words.
+//     tile's (probe row, build row) pairs in shared memory in output order
+//     and writes them column by column: neighbouring threads write neighbouring
+//     output rows, so stores are coalesced, and a warp owns whole validity
+//     words. Tiles of more than kWindow output rows are emit_long_kernel's,
+//     launched when the scan has seen one.
 // The lookup is bound by the latency of its dependent random reads (slot,
 // build key, chain link), so it keeps few registers and many warps, with no
 // barrier or atomic between the reads; the emission is bound by the build
@@ -683,7 +684,8 @@ __global__ void __launch_bounds__(kProbeThreads, kLookupBlocks) lookup_kernel(Pr
 }
 
 // Every tile's first output row (an exclusive scan of the tiles' rows, in
-// place); out[0] (mapped host memory): all rows, out[1]: the status word.
+// place); out[0] (mapped host memory): all rows, out[1]: the status word,
+// out[2]: whether a tile has more than kWindow output rows.
 constexpr int kScanThreads = 1024;
 __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(unsigned long long *tiles, int64_t n,
                                                                  const uint32_t *status, volatile unsigned long long *out) {
@@ -691,6 +693,7 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(unsigned long l
     constexpr int kPer = 16;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long run = 0;
+    bool large = false;
     for (int64_t t0 = 0; t0 < n; t0 += kScanThreads * kPer) {
         unsigned long long v[kPer], mine = 0;
         const int64_t i0 = t0 + (int64_t)threadIdx.x * kPer;
@@ -705,7 +708,10 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(unsigned long l
             for (int j = 0; j < kPer; j++) v[j] = i0 + j < n ? tiles[i0 + j] : 0;
         }
 #pragma unroll
-        for (int j = 0; j < kPer; j++) mine += v[j];
+        for (int j = 0; j < kPer; j++) {
+            mine += v[j];
+            large = large || v[j] > kWindow;
+        }
         unsigned long long incl = mine;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -735,9 +741,11 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(unsigned long l
         run += s_run;
         __syncthreads();  // s_warp and s_run are rewritten by the next chunk
     }
+    large = __syncthreads_or(large);
     if (threadIdx.x == 0) {
         out[0] = run;
         out[1] = status ? *status : 0u;
+        out[2] = large;
     }
 }
 
@@ -751,21 +759,23 @@ struct EmitDev {
     int pad;
 };
 
-// One output column of a window's m pairs (output rows first .. first + m),
-// by the whole CTA: four pairs' loads, then their stores. `rows`: the pairs'
-// rows of the column's side (kNone: NULL). With validity words a warp starts
-// at a multiple of 32 output rows and owns whole words but the window's ends.
-template <class T, class R>
+// One output column of m staged pairs (output rows first .. first + m), by N
+// threads: the CTA or a warp of it. Four pairs' loads, then their stores.
+// `rows`: the pairs' rows of the column's side (kNone: NULL). With validity
+// words a warp starts at a multiple of 32 output rows and owns whole words but
+// the ends.
+template <int N, class T, class R>
 __device__ __forceinline__ void emit_column(const OutColDev &c, const R *rows, int64_t base, unsigned long long first, int m) {
     constexpr int V = 4;
+    const int t = (int)threadIdx.x & (N - 1);
     const T *src = static_cast<const T *>(c.src) + (c.side == 0 ? base : 0);
     T *dst = static_cast<T *>(c.dst) + first;
     if (!c.dst_valid) {
-        for (int q0 = threadIdx.x; q0 < m; q0 += V * kProbeThreads) {
+        for (int q0 = t; q0 < m; q0 += V * N) {
             T v[V];
 #pragma unroll
             for (int j = 0; j < V; j++) {
-                const int q = q0 + j * kProbeThreads;
+                const int q = q0 + j * N;
                 v[j] = T{};
                 if (q >= m) continue;
                 const uint32_t r = rows[q];
@@ -773,12 +783,12 @@ __device__ __forceinline__ void emit_column(const OutColDev &c, const R *rows, i
             }
 #pragma unroll
             for (int j = 0; j < V; j++)
-                if (q0 + j * kProbeThreads < m) dst[q0 + j * kProbeThreads] = v[j];
+                if (q0 + j * N < m) dst[q0 + j * N] = v[j];
         }
         return;
     }
     const int64_t voff = c.src_voff + (c.side == 0 ? base : 0);
-    for (int q0 = (int)threadIdx.x - (int)(first & 31); q0 - (int)threadIdx.x < m; q0 += kProbeThreads) {
+    for (int q0 = t - (int)(first & 31); q0 - t < m; q0 += N) {
         const uint32_t r = (unsigned)q0 < (unsigned)m ? (uint32_t)rows[q0] : kNone;
         const bool some = (unsigned)q0 < (unsigned)m && (sizeof(R) == 2 || r != kNone);
         if ((unsigned)q0 < (unsigned)m) dst[q0] = some ? src[r] : T{};
@@ -787,34 +797,45 @@ __device__ __forceinline__ void emit_column(const OutColDev &c, const R *rows, i
             const int first_lane = q0 - (int)lane_id();  // the word's first pair
             uint32_t *p = c.dst_valid + ((unsigned long long)((long long)first + q0) >> 5);
             if (first_lane >= 0 && first_lane + 32 <= m) *p = w;
-            else atomicOr(p, w);  // a word shared with the next window or tile (zeroed before)
+            else atomicOr(p, w);  // a word shared with other pairs (zeroed before)
         }
     }
 }
-template <class R>
+template <int N, class R>
 __device__ __forceinline__ void emit_by_width(const OutColDev &c, const R *rows, int64_t base, unsigned long long first, int m) {
-    if (c.width == 8) emit_column<uint64_t>(c, rows, base, first, m);
-    else if (c.width == 4) emit_column<uint32_t>(c, rows, base, first, m);
-    else if (c.width == 16) emit_column<uint4>(c, rows, base, first, m);
-    else emit_column<uint8_t>(c, rows, base, first, m);
+    if (c.width == 8) emit_column<N, uint64_t>(c, rows, base, first, m);
+    else if (c.width == 4) emit_column<N, uint32_t>(c, rows, base, first, m);
+    else if (c.width == 16) emit_column<N, uint4>(c, rows, base, first, m);
+    else emit_column<N, uint8_t>(c, rows, base, first, m);
+}
+// All columns of m staged pairs, by N threads.
+template <int N>
+__device__ __forceinline__ void emit_pairs(const OutDev &out, const uint16_t *prow, const uint32_t *brow, int64_t base,
+                                           unsigned long long first, unsigned m) {
+    for (int k = 0; k < out.n; k++) {
+        const OutColDev c = out.c[k];
+        if (c.side == 0) {
+            emit_by_width<N>(c, prow, base, first, (int)m);
+        } else if (c.side == 1) {
+            emit_by_width<N>(c, brow, base, first, (int)m);
+        } else {  // the row index itself (3 probe, 4 build)
+            for (unsigned q = threadIdx.x & (N - 1); q < m; q += N)
+                static_cast<long long *>(c.dst)[first + q] =
+                    c.side == 3 ? (long long)(base + prow[q]) : brow[q] != kNone ? (long long)brow[q] : -1ll;
+        }
+    }
 }
 
-template <bool FILT, int LOOK>
-__global__ void __launch_bounds__(kProbeThreads, kEmitBlocks) emit_kernel(EmitDev E, OutDev out, FilterDev F) {
+// This thread's rows of its tile (neighbours, so that output order is probe
+// order): their first build rows and numbers of output rows, the output rows
+// before them in the tile, and the tile's. All threads of the CTA.
+template <int LOOK, class Sum>
+__device__ __forceinline__ void emit_rows(const EmitDev &E, int64_t tile, uint32_t (&cur)[kEmitRows], uint32_t (&cnt)[kEmitRows],
+                                          Sum *s_warp, Sum &before, Sum &total) {
     constexpr int U = kEmitRows, kWarps = kProbeThreads / 32;
-    // a tile's output rows: at most one per probe row, or chains of any length
-    using Sum = std::conditional_t<LOOK == kChains, unsigned long long, uint32_t>;
     static_assert(U == 4, "heads are read four at a time");
-    __shared__ Sum s_warp[kWarps];
-    __shared__ uint32_t s_brow[kWindow];
-    __shared__ uint16_t s_prow[kWindow];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t t0 = (int64_t)blockIdx.x * kTileRows;
-    const int64_t base = E.row0 + t0;  // the tile's first probe row
-    const int64_t l0 = t0 + threadIdx.x * U;
-    // neighbouring rows per thread: output order is probe order
-    const unsigned long long run = E.tiles[blockIdx.x];
-    uint32_t cur[U], cnt[U];
+    const int64_t l0 = tile * kTileRows + threadIdx.x * U;
     if (l0 + U <= E.rows) {
         const uint4 h = *reinterpret_cast<const uint4 *>(E.head + l0);
         cur[0] = h.x, cur[1] = h.y, cur[2] = h.z, cur[3] = h.w;
@@ -844,84 +865,120 @@ __global__ void __launch_bounds__(kProbeThreads, kEmitBlocks) emit_kernel(EmitDe
     }
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
-    Sum total = 0, before = 0;
+    total = 0;
+    before = incl - mine;
 #pragma unroll
     for (int w = 0; w < kWarps; w++) {
         const Sum c = s_warp[w];
         before += w < warp ? c : 0;
         total += c;
     }
-    // staged pairs, a window of the tile's output at a time
-    Sum at = before + (incl - mine);
-    int ru = 0;  // this thread's row being staged
-    uint32_t left = cnt[0], b = cur[0];
-    for (Sum w0 = 0; w0 < total; w0 += kWindow) {
-        const unsigned m = total - w0 < kWindow ? (unsigned)(total - w0) : (unsigned)kWindow;
-        if (LOOK == kChains && total <= kWindow) {
-            // the chains of the thread's rows side by side: each step is a
-            // dependent random read
-            uint32_t off[U], r[U];
-            bool more = true;
+}
+
+// The tiles of at most kWindow output rows, each staged whole.
+template <bool FILT, int LOOK>
+__global__ void __launch_bounds__(kProbeThreads, kEmitBlocks) emit_kernel(EmitDev E, OutDev out, FilterDev F) {
+    constexpr int U = kEmitRows;
+    // a tile's output rows: at most one per probe row, or chains of any length
+    using Sum = std::conditional_t<LOOK == kChains, unsigned long long, uint32_t>;
+    __shared__ Sum s_warp[kProbeThreads / 32];
+    __shared__ uint32_t s_brow[kWindow];
+    __shared__ uint16_t s_prow[kWindow];
+    const int64_t base = E.row0 + (int64_t)blockIdx.x * kTileRows;  // the tile's first probe row
+    uint32_t cur[U], cnt[U];
+    Sum before, total;
+    emit_rows<LOOK>(E, blockIdx.x, cur, cnt, s_warp, before, total);
+    if (LOOK == kChains && total > kWindow) return;  // emit_long_kernel's
+    uint32_t at = (uint32_t)before;
+    if (LOOK == kChains) {
+        // the chains of the thread's rows side by side: each step is a
+        // dependent random read
+        uint32_t off[U];
+        bool more = true;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            off[u] = at;
+            at += cnt[u];
+        }
+        for (uint32_t k = 0; more; k++) {
+            more = false;
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                off[u] = (uint32_t)at;
-                at += cnt[u];
-                r[u] = cur[u];
+                if (k >= cnt[u]) continue;
+                s_prow[off[u] + k] = (uint16_t)(threadIdx.x * U + u);
+                s_brow[off[u] + k] = cur[u];
+                if (k + 1 >= cnt[u]) continue;
+                cur[u] = __ldg(E.next + cur[u]);
+                if (FILT) cur[u] = first_true(F, base + threadIdx.x * U + u, cur[u], E.next);
+                more = true;
             }
-            for (uint32_t k = 0; more; k++) {
-                more = false;
+        }
+    } else {
 #pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (k >= cnt[u]) continue;
-                    s_prow[off[u] + k] = (uint16_t)(threadIdx.x * U + u);
-                    s_brow[off[u] + k] = r[u];
-                    if (k + 1 >= cnt[u]) continue;
-                    r[u] = __ldg(E.next + r[u]);
-                    if (FILT) r[u] = first_true(F, base + threadIdx.x * U + u, r[u], E.next);
-                    more = true;
-                }
-            }
-        } else if (LOOK == kChains) {
-            while (at < w0 + m) {
-                while (left == 0 && ru < U - 1) {
-                    ru++;
-#pragma unroll
-                    for (int u = 1; u < U; u++)
-                        if (u == ru) left = cnt[u], b = cur[u];
-                }
-                if (left == 0) break;  // every row of this thread is staged
-                s_prow[at - w0] = (uint16_t)(threadIdx.x * U + ru);
-                s_brow[at - w0] = b;
-                at++;
+        for (int u = 0; u < U; u++) {
+            if (!cnt[u]) continue;
+            s_prow[at] = (uint16_t)(threadIdx.x * U + u);
+            s_brow[at] = cur[u];
+            at++;
+        }
+    }
+    __syncthreads();
+    emit_pairs<kProbeThreads>(out, s_prow, s_brow, base, E.tiles[blockIdx.x], (unsigned)total);
+}
+
+// The tiles of more than kWindow output rows (long chains of duplicate build
+// keys), kLongParts CTAs to a tile and each warp for itself: its lanes follow
+// their rows' chains side by side, a step at a time, stage the pairs as they come
+// and write them out whenever the warp's share of the window may not hold
+// another step. Bound by the chains' dependent reads. Measured on B200, 50,000
+// probe rows, chains of 1,024, 25M output rows of three columns: 0.67 ms (the
+// join 1.9 ms; 2.9 with four rows to a lane). With the CTA staging a window of
+// its tile at a time, only the threads whose rows fell into it followed chains,
+// and the join took 92 ms; a warp per 32 rows writing each step took 2.0 ms.
+constexpr int kLongParts = kTileRows / kProbeThreads;
+template <bool FILT>
+__global__ void __launch_bounds__(kProbeThreads) emit_long_kernel(EmitDev E, OutDev out, FilterDev F) {
+    constexpr int kWarps = kProbeThreads / 32, kShare = kWindow / kWarps;
+    static_assert(kShare >= 64, "a warp's share holds more than a step's pairs");
+    __shared__ unsigned long long s_warp[kWarps], s_before[kProbeThreads];
+    __shared__ uint32_t s_brow[kWarps][kShare];
+    __shared__ uint16_t s_prow[kWarps][kShare];
+    const int warp = threadIdx.x >> 5;
+    const int64_t tile = blockIdx.x / kLongParts;
+    const int part = blockIdx.x % kLongParts * kProbeThreads;  // this CTA's first row of the tile
+    const int64_t base = E.row0 + tile * kTileRows;
+    unsigned long long first;
+    {
+        uint32_t cur[kEmitRows], cnt[kEmitRows];
+        unsigned long long before, total;
+        emit_rows<kChains>(E, tile, cur, cnt, s_warp, before, total);
+        if (total <= kWindow) return;  // emit_kernel's
+        s_before[threadIdx.x] = before;  // the output rows before tile row threadIdx.x * kEmitRows
+        __syncthreads();
+        first = E.tiles[tile] + s_before[(part + warp * 32) / kEmitRows];
+    }
+    const int row = part + (int)threadIdx.x;
+    const bool live = tile * kTileRows + row < E.rows;
+    uint32_t cur = live ? E.head[tile * kTileRows + row] : kNone, left = live ? E.cnt[tile * kTileRows + row] : 0;
+    unsigned want = __ballot_sync(kFull, left != 0);
+    while (want) {
+        unsigned m = 0;
+        for (; want && m + 32 <= (unsigned)kShare; want = __ballot_sync(kFull, left != 0)) {
+            if (left) {
+                const unsigned q = m + __popc(want & lanemask_lt());
+                s_prow[warp][q] = (uint16_t)row;
+                s_brow[warp][q] = cur;
                 if (--left) {
-                    b = __ldg(E.next + b);
-                    if (FILT) b = first_true(F, base + threadIdx.x * U + ru, b, E.next);
+                    cur = __ldg(E.next + cur);
+                    if (FILT) cur = first_true(F, base + row, cur, E.next);
                 }
             }
-        } else {
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (!cnt[u]) continue;
-                s_prow[at] = (uint16_t)(threadIdx.x * U + u);
-                s_brow[at] = cur[u];
-                at++;
-            }
+            m += __popc(want);
         }
-        __syncthreads();
-        const unsigned long long first = run + w0;
-        for (int k = 0; k < out.n; k++) {
-            const OutColDev c = out.c[k];
-            if (c.side == 0) {
-                emit_by_width(c, s_prow, base, first, (int)m);
-            } else if (c.side == 1) {
-                emit_by_width(c, s_brow, base, first, (int)m);
-            } else {  // the row index itself (3 probe, 4 build)
-                for (unsigned q = threadIdx.x; q < m; q += kProbeThreads)
-                    static_cast<long long *>(c.dst)[first + q] =
-                        c.side == 3 ? (long long)(base + s_prow[q]) : s_brow[q] != kNone ? (long long)s_brow[q] : -1ll;
-            }
-        }
-        __syncthreads();
+        __syncwarp();
+        emit_pairs<32>(out, s_prow[warp], s_brow[warp], base, first, m);
+        first += m;
+        __syncwarp();  // the share is staged anew
     }
 }
 
@@ -1579,9 +1636,16 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
         rt_->launches++;
         check_launch("lookup_kernel");
     };
+    bool long_tiles = false;  // tiles of more than kWindow output rows (known once the total is)
     auto launch_emit = [&](int look, const EmitDev &E, const OutDev &od) {
         if (E.rows == 0 || od.n == 0) return;
         const int grid = (int)ceil_div(E.rows, kTileRows);
+        if (long_tiles) {
+            if (filt) emit_long_kernel<true><<<grid * kLongParts, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
+            else emit_long_kernel<false><<<grid * kLongParts, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
+            rt_->launches++;
+            check_launch("emit_long_kernel");
+        }
         if (look == kChains && filt) emit_kernel<true, kChains><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
         else if (look == kChains) emit_kernel<false, kChains><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
         else if (look == kRowsOnly) emit_kernel<false, kRowsOnly><<<grid, kProbeThreads, 0, rt_->stream>>>(E, od, fd);
@@ -1703,6 +1767,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
             reinterpret_cast<volatile unsigned long long *>(static_cast<uint8_t *>(rt_->status_host) + 64);
         if (seen[1] & ST_TOO_MANY)
             fail(KRV_TOO_MANY_ROWS, "SCALAR_SUBQUERY_TOO_MANY_ROWS: a probe row matched more than one build row");
+        long_tiles = seen[2] != 0;
         return (int64_t)seen[0];
     };
     // The output columns for m rows, and the kernel that fills them.
