@@ -1604,7 +1604,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
         A.dir = DirectDev{direct_.as<uint32_t>(), key_lo_, direct_span_};
         A.marks = marks;
         A.pad = pad;
-        A.single_match = spec_.single_match;
+        A.single_match = status ? spec_.single_match : 0;
         A.kind = kind;
         A.build_empty = build_rows_ == 0;
         A.build_has_null = any_null_build_;
@@ -1730,6 +1730,16 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     const int64_t ntiles = ceil_div(n, (int64_t)kTileRows);
     DBuf head, cnt, tiles, status;
     int64_t chunk = n;  // rows looked up and emitted together
+    bool kept = true;   // every row's lookup is kept until it is emitted
+    // Otherwise rows are looked up again, a chunk at a time, when they are emitted.
+    auto keep_a_chunk = [&] {
+        kept = false;
+        head = DBuf();
+        cnt = DBuf();
+        chunk = std::min(n, std::min<int64_t>(64, ceil_div(ntiles, (int64_t)64)) * kTileRows);
+        head = DBuf(rt_, (size_t)chunk * 4);
+        if (how == kChains) cnt = DBuf(rt_, (size_t)chunk * 4);
+    };
     if (!none) {
         if (spec_.single_match) {
             status = DBuf(rt_, 8);
@@ -1741,12 +1751,8 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
             if (how == kChains) cnt = DBuf(rt_, (size_t)n * 4);
         } catch (const Error &e) {
             if (e.code != KRV_NEED_MEMORY) throw;
-            // No room to keep every row's lookup: count now, and look up
-            // again, a chunk at a time, when the rows are emitted.
-            head = DBuf();
-            chunk = std::min<int64_t>(n, 64 * kTileRows);
+            keep_a_chunk();
         }
-        const bool kept = head.get() != nullptr;
         launch_lookup(how, 0, n, kept ? head.as<uint32_t>() : nullptr, kept && how == kChains ? cnt.as<uint32_t>() : nullptr,
                       tiles.as<unsigned long long>(), pairs ? marks : nullptr, pads && pairs, kind, status.as<uint32_t>());
         tile_scan_kernel<<<1, kScanThreads, 0, rt_->stream>>>(
@@ -1754,10 +1760,6 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
             reinterpret_cast<volatile unsigned long long *>(static_cast<uint8_t *>(rt_->status_host_dev) + 64));
         rt_->launches++;
         check_launch("tile_scan_kernel");
-        if (!kept) {
-            head = DBuf(rt_, (size_t)chunk * 4);
-            if (how == kChains) cnt = DBuf(rt_, (size_t)chunk * 4);
-        }
     }
     auto total = [&]() -> int64_t {  // waits for the scan
         if (none) return 0;
@@ -1813,7 +1815,7 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
         if (m == 0 || none) return;
         for (int64_t row0 = 0; row0 < n; row0 += chunk) {
             const int64_t rows = std::min(chunk, n - row0);
-            if (chunk < n)
+            if (!kept)
                 launch_lookup(how, row0, rows, head.as<uint32_t>(), how == kChains ? cnt.as<uint32_t>() : nullptr, nullptr,
                               nullptr, pads && pairs, kind, nullptr);
             E.row0 = row0;
@@ -1843,8 +1845,21 @@ DevBatch HashJoin::probe(const DevBatch &outer_in) {
     } else {
         m = total();
     }
-    if (m < 0) m = total();
-    else emit(m);
+    if (m < 0) {
+        m = total();
+    } else {
+        try {
+            emit(m);
+        } catch (const Error &e) {
+            // the lookups' memory may be what the output lacks
+            if (e.code != KRV_NEED_MEMORY || none || !kept) throw;
+            out = DevBatch{};
+            idx[0] = DBuf();
+            idx[1] = DBuf();
+            keep_a_chunk();
+            emit(m);
+        }
+    }
     out.rows = m;
     for (DevCol &c : out.cols) c.length = m;
     for (const VarOut &v : vars) {

@@ -96,3 +96,29 @@ def test_a_slice_that_cannot_be_handed_out_waits(kb, small, call):
         st = take(more)
     assert failed >= 3 and sorted(rows) == (k.tolist() if call == "probe" else (build * 3).tolist())
     j.close()
+
+
+@pytest.mark.parametrize("dup,jt", [(1, "left_outer"), (1, "left_semi"), (2, "inner"), (2, "left_outer")])
+@pytest.mark.parametrize("n", [1_000_003, 50_003])
+def test_probe_with_room_for_little_but_its_output(kb, small, dup, jt, n):
+    nb = 100_003
+    k = np.random.default_rng(dup).permutation(nb).astype(np.int64) * 1_000_003
+    pk = np.random.default_rng(n).permutation(np.resize(k, n))
+    semi = jt == "left_semi"
+    j = kb.HashJoin(small, kb.join_spec(jt, probe_out=[0, 1], build_out=[] if semi else [1]))
+    j.build_push_device(kb.DeviceBatch([column("k", np.tile(k, dup)), column("v", np.arange(nb * dup))]))
+    j.build_finish()
+    p = kb.DeviceBatch([column("k", pk), column("r", np.arange(n))])
+    out_rows = n * dup
+    out = out_rows * (16 if semi else 24) + (out_rows // 8 if jt == "left_outer" else 0)
+    b = ballast(kb, small, BUDGET, out + n // 8 + (96 << 10))  # less than the rows' lookups take
+    r = j.probe_device(p)
+    b.close()
+    assert r.rows == out_rows
+    row = r.columns[1].cpu().numpy()
+    assert np.array_equal(np.sort(row), np.repeat(np.arange(n), dup))
+    assert np.array_equal(r.columns[0].cpu().numpy(), pk[row])
+    if not semi:
+        v = r.columns[2].cpu().numpy()
+        assert np.array_equal(k[v % nb], pk[row]) and np.unique(row * (nb * dup) + v).size == out_rows
+    j.close()
