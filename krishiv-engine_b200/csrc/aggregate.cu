@@ -2148,6 +2148,7 @@ class HashAggregate {
 
   public:
     ~HashAggregate() {
+        give_spare_back();
         if (dict_) key_dict_destroy(dict_);
         for (KeyDict *d : vdicts_)
             if (d) key_dict_destroy(d);
@@ -2190,6 +2191,14 @@ class HashAggregate {
     // inserts them before anything looks keys up or rehashes the table.
     int64_t unindexed_from_ = -1;
     void index_pending();
+    // What the table takes beyond the size hint, counted in the runtime's pool
+    // (which outlives the runtime).
+    int64_t spare_bytes_ = 0;
+    std::shared_ptr<Pool> pool_;
+    void give_spare_back() {
+        if (pool_) pool_->spare.fetch_sub(spare_bytes_);
+        pool_.reset();
+    }
     // agg_fold_kernel's bound on new group ids: the table's limit, less the
     // ids that the resident CTAs may take past a check they passed together.
     uint64_t part_id_room(int part_blocks) const { return (uint64_t)part_blocks * rt_->sm_count * (uint64_t)fold_cap_; }
@@ -2444,13 +2453,31 @@ void HashAggregate::plan(const DevBatch &b) {
     plan_row_records();
     const uint64_t hint = spec_.expected_groups > 0 ? (uint64_t)spec_.expected_groups : 65536;
     uint64_t slots = std::max<uint64_t>(1024, next_pow2((uint64_t)(hint * 2)));
-    // A small hint does not make a small table where memory is no matter: the
-    // batches that could not fill it are not asked how many groups they had
-    // (on B200 100,000 rows in 13 batches, hint 1000: 0.34 ms, 0.51 with
-    // the table of 2048 slots).
+    // A small hint does not make a small table where no budget limits the
+    // runtime: the batches that could not fill it are not asked how many groups
+    // they had (on B200 100,000 rows in 13 batches, hint 1000: 0.34 ms, 0.51
+    // with the table of 2048 slots). All of a runtime's aggregates together take
+    // at most kSpareBytes more than their hints that way.
     constexpr uint64_t kMinSlots = 1 << 17;
-    if (rt_->budget == 0 || kMinSlots * (uint64_t)(P_.rec + 20) <= (uint64_t)rt_->budget / 64) slots = std::max(slots, kMinSlots);
-    alloc_table(slots);
+    constexpr int64_t kSpareBytes = 1ll << 30;
+    const int64_t more = slots < kMinSlots ? (int64_t)((kMinSlots - slots) * (uint64_t)(P_.rec + 20)) : 0;
+    bool spare = more > 0 && rt_->budget == 0;
+    if (spare && rt_->pool->spare.fetch_add(more) + more > kSpareBytes) {
+        rt_->pool->spare.fetch_sub(more);
+        spare = false;
+    }
+    if (spare) {
+        pool_ = rt_->pool;
+        spare_bytes_ = more;
+        try {
+            alloc_table(kMinSlots);
+        } catch (const Error &e) {
+            if (e.code != KRV_NEED_MEMORY) throw;
+            give_spare_back();
+            spare = false;
+        }
+    }
+    if (!spare) alloc_table(slots);
     planned_ = true;
 }
 

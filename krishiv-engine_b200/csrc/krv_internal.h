@@ -47,6 +47,7 @@ struct Pool {
     cudaStream_t stream = nullptr;
     int device = 0;
     std::atomic<bool> alive{true};
+    std::atomic<int64_t> spare{0};  // of `used`: what aggregates' tables take beyond their size hints
 };
 
 // Page-locked host blocks kept for reuse: the spill space of partitioned
