@@ -2125,7 +2125,8 @@ class HashAggregate {
 
   private:
     void plan(const DevBatch &b);
-    void alloc_table(uint64_t slots);
+    void alloc_table(uint64_t slots, DBuf &okeys, DBuf &ogids);
+    void unplan();
     void grow(uint64_t need_groups);
     void launch(const DevBatch &b, const KeyIn &key, int64_t n, const uint32_t *rows_idx, uint32_t *ovf,
                 unsigned long long *ovf_count);
@@ -2147,12 +2148,7 @@ class HashAggregate {
     std::vector<std::pair<int, int>> poison_src_;
 
   public:
-    ~HashAggregate() {
-        give_spare_back();
-        if (dict_) key_dict_destroy(dict_);
-        for (KeyDict *d : vdicts_)
-            if (d) key_dict_destroy(d);
-    }
+    ~HashAggregate() { unplan(); }
 
   private:
     AggPlanDev P_{};
@@ -2461,6 +2457,7 @@ void HashAggregate::plan(const DevBatch &b) {
     constexpr uint64_t kMinSlots = 1 << 17;
     constexpr int64_t kSpareBytes = 1ll << 30;
     const int64_t more = slots < kMinSlots ? (int64_t)((kMinSlots - slots) * (uint64_t)(P_.rec + 20)) : 0;
+    DBuf none;  // no table before
     bool spare = more > 0 && rt_->budget == 0;
     if (spare && rt_->pool->spare.fetch_add(more) + more > kSpareBytes) {
         rt_->pool->spare.fetch_sub(more);
@@ -2470,38 +2467,44 @@ void HashAggregate::plan(const DevBatch &b) {
         pool_ = rt_->pool;
         spare_bytes_ = more;
         try {
-            alloc_table(kMinSlots);
+            alloc_table(kMinSlots, none, none);
         } catch (const Error &e) {
             if (e.code != KRV_NEED_MEMORY) throw;
             give_spare_back();
             spare = false;
         }
     }
-    if (!spare) alloc_table(slots);
+    if (!spare) alloc_table(slots, none, none);
     planned_ = true;
 }
 
-void HashAggregate::alloc_table(uint64_t slots) {
-    slots_ = slots;
-    limit_ = (unsigned long long)(slots * 3 / 4);
-    keys_ = DBuf(rt_, slots * 8);
-    gids_ = DBuf(rt_, slots * 4);
-    KRV_CUDA(cudaMemsetAsync(keys_.get(), 0x80, slots * 8, rt_->stream));
-    KRV_CUDA(cudaMemsetAsync(gids_.get(), 0xFF, slots * 4, rt_->stream));
+// A table of `slots` slots with the records of the one before, whose slots
+// (left in okeys and ogids) the caller puts in again. All or nothing: without
+// memory for it the table stays as it is.
+void HashAggregate::alloc_table(uint64_t slots, DBuf &okeys, DBuf &ogids) {
     const size_t gcap = slots + kFirstGid;
-    DBuf states(rt_, gcap * (size_t)P_.rec);
-    DBuf gkeys(rt_, gcap * 8);
+    DBuf keys(rt_, slots * 8), gids(rt_, slots * 4), states(rt_, gcap * (size_t)P_.rec), gkeys(rt_, gcap * 8);
+    DBuf ctl_buf;
+    if (!states_.get()) ctl_buf = DBuf(rt_, sizeof(AggCtl));
+    KRV_CUDA(cudaMemsetAsync(keys.get(), 0x80, slots * 8, rt_->stream));
+    KRV_CUDA(cudaMemsetAsync(gids.get(), 0xFF, slots * 4, rt_->stream));
     if (states_.get()) {
         KRV_CUDA(cudaMemcpyAsync(states.get(), states_.get(), (size_t)known_groups_ * P_.rec, cudaMemcpyDeviceToDevice,
                                  rt_->stream));
         KRV_CUDA(cudaMemcpyAsync(gkeys.get(), gkeys_.get(), (size_t)known_groups_ * 8, cudaMemcpyDeviceToDevice,
                                  rt_->stream));
     } else {
-        ctl_ = DBuf(rt_, sizeof(AggCtl));
+        ctl_ = std::move(ctl_buf);
         init_special_kernel<<<1, 32, 0, rt_->stream>>>(P_, states.as<uint8_t>(), ctl());
         rt_->launches++;
         check_launch("init_special_kernel");
     }
+    slots_ = slots;
+    limit_ = (unsigned long long)(slots * 3 / 4);
+    okeys = std::move(keys_);
+    ogids = std::move(gids_);
+    keys_ = std::move(keys);
+    gids_ = std::move(gids);
     states_ = std::move(states);
     gkeys_ = std::move(gkeys);
 }
@@ -2525,10 +2528,10 @@ TableDev HashAggregate::table() const {
 void HashAggregate::grow(uint64_t need_groups) {
     // the records to carry over: every group the device has handed out
     if (pending_rows_) read_ctl();
-    DBuf okeys = std::move(keys_), ogids = std::move(gids_);
+    DBuf okeys, ogids;
     const uint64_t oslots = slots_;
     uint64_t ns = next_pow2(std::max<uint64_t>(oslots * 2, need_groups * 2));
-    alloc_table(ns);
+    alloc_table(ns, okeys, ogids);
     rehash_kernel<<<grid_for(rt_, (int64_t)oslots, 256, 8), 256, 0, rt_->stream>>>(
         okeys.as<long long>(), ogids.as<uint32_t>(), oslots, keys_.as<long long>(), gids_.as<uint32_t>(), slots_ - 1);
     rt_->launches++;
@@ -2808,7 +2811,6 @@ void HashAggregate::plan_row_records() {
 }
 
 void HashAggregate::plan_partitioned(const KeyIn &key, int64_t n) {
-    part_planned_ = true;
     // The sample: a strided 64K rows of the first large batch.
     const int m = (int)std::min<int64_t>(n, kPartSample);
     // Hot: keys of at least kHotRows rows by the sample. Every CTA of the
@@ -2849,6 +2851,7 @@ void HashAggregate::plan_partitioned(const KeyIn &key, int64_t n) {
     const int64_t d = std::max<int64_t>(0, (int64_t)c.distinct - part_hot_), f1 = c.singles;
     const double est = (double)d + (double)f1 * (std::sqrt((double)n / std::max(1, m)) - 1.0);
     part_groups_est_ = std::max<int64_t>({(int64_t)est, spec_.expected_groups, 1});
+    part_planned_ = true;
 }
 
 void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_t n) {
@@ -3006,10 +3009,35 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
     }
 }
 
+// Undoes plan(), whole or begun.
+void HashAggregate::unplan() {
+    give_spare_back();
+    if (dict_) key_dict_destroy(dict_);
+    dict_ = nullptr;
+    for (KeyDict *d : vdicts_)
+        if (d) key_dict_destroy(d);
+    vdicts_.clear();
+    dict_cols_.clear();
+    expr_col_.clear();
+    expr_aux_.clear();
+    poison_src_.clear();
+    value_cols_.clear();
+    input_types_.clear();
+    input_names_.clear();
+    mode_ = spec_.mode == KRV_AGG_MODE_GLOBAL ? KRV_AGG_MODE_GLOBAL : KRV_AGG_MODE_SHARED;
+}
+
 void HashAggregate::push(const DevBatch &in) {
     if (finished_) fail(KRV_INVALID_ARGUMENT, "push after finish");
     DeviceGuard g(rt_);
-    if (!planned_) plan(in);
+    if (!planned_) {
+        try {
+            plan(in);
+        } catch (...) {
+            unplan();  // the next push plans anew
+            throw;
+        }
+    }
     if (in.cols.size() != input_types_.size()) fail(KRV_INVALID_ARGUMENT, "batches differ in columns");
     for (size_t i = 0; i < in.cols.size(); i++)
         if (in.cols[i].type != input_types_[i]) fail(KRV_INVALID_ARGUMENT, "batches differ in types");

@@ -38,3 +38,40 @@ def test_many_small_aggregates_live_together(kb, rt, budget):
     small.synchronize()
     assert small.used_bytes < 1 << 20
     small.close()
+
+
+@pytest.mark.parametrize("keys", [1, 2])
+def test_push_that_finds_no_memory_may_be_made_again(kb, rt, keys):
+    from test_join_memory_gpu import ballast, status
+    budget = 512 << 20
+    small = kb.Runtime.on_torch_stream(0, budget_bytes=budget, stream=rt.torch_stream)
+    rng = np.random.default_rng(keys)
+    n, groups = 300_001, 150_000  # more groups than the hint's table, and rows enough for the partitioned kernels
+    k, v = rng.integers(0, groups, n), rng.integers(-99, 99, n)
+    cols = [("k", torch.as_tensor(k, device="cuda"), None)]
+    if keys == 2:
+        cols = [("k0", (cols[0][1] // 400).to(torch.int32), None), ("k1", (cols[0][1] % 400).to(torch.int32), None)]
+    cols.append(("v", torch.as_tensor(v, device="cuda"), None))
+    batch = kb.DeviceBatch(cols)
+    a = kb.HashAggregate(small, kb.agg_spec(0 if keys == 1 else (0, 1), [("sum", keys), ("count_star", 0)], expected_groups=10))
+    failed = 0
+    for free in [1 << 14] + [i << 21 for i in range(1, 100)]:
+        b = ballast(kb, small, budget, free)
+        st = status(kb, a.push_device, batch)
+        if b is not None:
+            b.close()
+        if st == kb.OK:
+            break
+        assert st == kb.NEED_MEMORY
+        failed += 1
+    assert failed > 2 and st == kb.OK
+    a.finish()
+    r = a.result_device()
+    c = [x.cpu().numpy() for x in r.columns]
+    key = c[0] if keys == 1 else c[0].astype(np.int64) * 400 + c[1]
+    order = np.argsort(key)
+    assert np.array_equal(key[order], np.unique(k))
+    assert np.array_equal(c[keys][order], np.bincount(k, v, minlength=groups)[key[order]].astype(np.int64))
+    assert np.array_equal(c[keys + 1][order], np.bincount(k, minlength=groups)[key[order]])
+    a.close()
+    small.close()
