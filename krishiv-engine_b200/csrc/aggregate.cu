@@ -2931,12 +2931,12 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
                                                       &ctl()->cold);
         rt_->launches++;
         check_launch("part_bases_kernel");
-        // Room for the cold rows: for every row when that is little, else (or
-        // when there is no such room) for as many as were counted.
+        // Room for the cold rows: for every row when that is little and no budget
+        // limits the runtime, else (or when there is no such room) for as many
+        // as were counted.
         unsigned long long cold = (unsigned long long)ns;
         DBuf part_buf;
-        const uint64_t most = (uint64_t)ns * part_row_bytes_;
-        if (most <= kPartBufBytes && (rt_->budget == 0 || most <= (uint64_t)rt_->budget / 8)) {
+        if ((uint64_t)ns * part_row_bytes_ <= kPartBufBytes && rt_->budget == 0) {
             try {
                 part_buf = DBuf(rt_, (size_t)cold * part_row_bytes_);
             } catch (const Error &e) {

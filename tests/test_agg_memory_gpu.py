@@ -75,3 +75,23 @@ def test_push_that_finds_no_memory_may_be_made_again(kb, rt, keys):
     assert np.array_equal(c[keys + 1][order], np.bincount(k, minlength=groups)[key[order]])
     a.close()
     small.close()
+
+
+def test_large_batch_of_hot_keys_takes_little_memory(kb, rt):
+    """Nearly every row is of a key that the sample knows: under a budget the few others' partitions leave room for the table."""
+    from test_join_memory_gpu import ballast
+    budget = 512 << 20
+    small = kb.Runtime.on_torch_stream(0, budget_bytes=budget, stream=rt.torch_stream)
+    rng = np.random.default_rng(5)
+    n = 1_700_003  # 54 MB as partition rows
+    k, v = rng.integers(0, 100, n), rng.integers(-99, 99, n)
+    k[::100] = rng.integers(100, 20_000, k[::100].size)
+    a = kb.HashAggregate(small, kb.agg_spec(0, [("sum", 1), ("count_star", 0)], expected_groups=100))
+    b = ballast(kb, small, budget, 130 << 20)
+    push(kb, a, k, v)
+    b.close()
+    key, total, count = groups_of(a)
+    assert np.array_equal(key, np.unique(k))
+    assert np.array_equal(total, np.bincount(k, v)[key].astype(np.int64)) and np.array_equal(count, np.bincount(k)[key])
+    a.close()
+    small.close()
