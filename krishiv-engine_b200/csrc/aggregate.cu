@@ -1142,7 +1142,8 @@ struct FoldDev {
     const int *todo;   // the partitions to run: CTA b runs partition todo[b] (all, in order, when null)
     uint32_t *start;   // per partition: its first row not yet merged (read and written)
     int *failed;       // partitions that stopped for want of room in the global table
-    unsigned long long id_limit;  // new group ids only while the count is at most this
+    unsigned long long room;      // new groups that the table has room for
+    unsigned long long *claimed;  // new groups asked for by this launch
     int lookup;                   // the global table may hold keys of these partitions
 };
 constexpr uint32_t kNoGid = 0xFFFFFFFFu, kNewGid = 0x80000000u;
@@ -1292,9 +1293,9 @@ __global__ void __launch_bounds__(kFoldThreads, 3) agg_fold_kernel(AggPlanDev P,
             __syncthreads();
         }
         if (t == 0 && s_new) {  // ids for the new keys, all or none
-            // Checked, then added: CTAs that pass the check together take at
-            // most the ids past the limit that the table has room for.
-            if (__ldcg(T.ngroups) + (unsigned long long)s_new > D.id_limit) s_fail = 1;
+            // Claimed first, and a claim past the room is not taken back: the
+            // ids handed out are within the room and without a gap.
+            if (atomicAdd(D.claimed, (unsigned long long)s_new) + (unsigned long long)s_new > D.room) s_fail = 1;
             else s_base = atomicAdd(T.ngroups, (unsigned long long)s_new);
         }
         if (__syncthreads_or(s_fail)) {
@@ -1756,6 +1757,8 @@ struct AggCtl {
     uint32_t status, pad0;       // status bits; a set bit fails the aggregate, so it is never cleared
     unsigned long long deferred; // rows that found no room in the table
     unsigned long long cold;     // rows in the partitions
+    // of the fold kernel's launch (cleared together)
+    unsigned long long claimed;  // new groups asked for
     int32_t failed, pad1;        // partitions that stopped for want of room
     // the key sample (see hot_pick_kernel)
     uint32_t special, distinct, singles, runs, hot, hot_rows, hot_buckets, pad2;
@@ -2195,14 +2198,7 @@ class HashAggregate {
         if (pool_) pool_->spare.fetch_sub(spare_bytes_);
         pool_.reset();
     }
-    // agg_fold_kernel's bound on new group ids: the table's limit, less the
-    // ids that the resident CTAs may take past a check they passed together.
-    uint64_t part_id_room(int part_blocks) const { return (uint64_t)part_blocks * rt_->sm_count * (uint64_t)fold_cap_; }
     int fold_slots_ = 0, fold_cap_ = 0;  // agg_fold_kernel's local table (cap 0: records too large for it)
-    unsigned long long part_id_limit(int part_blocks) const {
-        const uint64_t room = part_id_room(part_blocks), cap = slots_ / 8 * 7;
-        return cap > room ? std::min<unsigned long long>(limit_, cap - room) : 0ull;
-    }
     // All sampled keys are hot: push_few may take the batch.
     bool few_keys_ = false;
     bool push_few(const DevBatch &b, const KeyIn &key, int64_t n);
@@ -2917,7 +2913,6 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
         // every CTA's share of each placed within it.
         DBuf cta_rows(rt_, (size_t)nparts * S.ctas * 4), totals(rt_, (size_t)nparts * 4);
         DBuf part_base(rt_, (size_t)(nparts + 1) * 4);
-        KRV_CUDA(cudaMemsetAsync(&ctl()->failed, 0, 4, rt_->stream));
         S.cta_rows = cta_rows.as<unsigned>();
         KRV_CUDA(cudaMemsetAsync(cta_rows.get(), 0, cta_rows.bytes(), rt_->stream));
         agg_count_kernel<<<2 * S.ctas, kSplitThreads, count_smem, rt_->stream>>>(ks, ns, S);
@@ -2951,8 +2946,11 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
         KRV_CUDA(cudaMemsetAsync(start.get(), 0, start.bytes(), rt_->stream));
         // Room in the table for the keys this slice may add (an estimate; a
         // partition that finds none stops and runs again after a grow).
+        // Without a budget there is room for a table's keys of every resident
+        // CTA beside, in case that the estimate is low.
         const int64_t want = known_groups_ + std::min<int64_t>(ns, part_groups_est_) + H + 2;
-        if (want > (int64_t)part_id_limit(part_blocks)) grow((uint64_t)want + part_id_room(part_blocks));
+        const int64_t beside = rt_->budget == 0 ? (int64_t)part_blocks * rt_->sm_count * fold_cap_ : 0;
+        if (want > (int64_t)limit_ || want + beside > (int64_t)(slots_ / 8 * 7)) grow((uint64_t)(want + beside));
         const TableDev T = table();
         S.part_buf = part_buf.as<uint8_t>();
         S.part_base = part_base.as<unsigned>();
@@ -2972,7 +2970,9 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
         D.todo = nullptr;
         D.start = start.as<uint32_t>();
         D.failed = &ctl()->failed;
-        D.id_limit = part_id_limit(part_blocks);
+        D.claimed = &ctl()->claimed;
+        D.room = limit_ - (unsigned long long)known_groups_;
+        KRV_CUDA(cudaMemsetAsync(&ctl()->claimed, 0, 16, rt_->stream));
         // Cold keys already in the table (from earlier batches or slices)
         // are looked up; the first slice's are all new.
         D.lookup = known_groups_ > (int64_t)kFirstGid + H ? 1 : 0;
@@ -2990,16 +2990,20 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
             KRV_CUDA(cudaMemcpyAsync(hb.data(), part_base.get(), hb.size() * 4, cudaMemcpyDeviceToHost, rt_->stream));
             KRV_CUDA(cudaStreamSynchronize(rt_->stream));
             std::vector<int> again;
+            int64_t left = 0;  // their rows
             for (int p = 0; p < nparts; p++)
-                if (hs[p] < hb[p + 1] - hb[p]) again.push_back(p);
-            grow((uint64_t)known_groups_ + (uint64_t)again.size() * (uint64_t)fold_cap_ + part_id_room(part_blocks) + 1);
+                if (hs[p] < hb[p + 1] - hb[p]) {
+                    again.push_back(p);
+                    left += hb[p + 1] - hb[p] - hs[p];
+                }
+            grow((uint64_t)(known_groups_ + std::min<int64_t>(left, (int64_t)again.size() * fold_cap_) + beside + 1));
             unindexed_from_ = known_groups_;  // grow indexed every group so far
             todo = DBuf(rt_, again.size() * 4);
             KRV_CUDA(cudaMemcpyAsync(todo.get(), again.data(), again.size() * 4, cudaMemcpyHostToDevice, rt_->stream));
-            KRV_CUDA(cudaMemsetAsync(&ctl()->failed, 0, 4, rt_->stream));
+            KRV_CUDA(cudaMemsetAsync(&ctl()->claimed, 0, 16, rt_->stream));
             const TableDev T2 = table();
             D.todo = todo.as<int>();
-            D.id_limit = part_id_limit(part_blocks);
+            D.room = limit_ - (unsigned long long)known_groups_;
             D.lookup = 1;
             agg_fold_kernel<<<(int)again.size(), kFoldThreads, part_smem, rt_->stream>>>(P, T2, D);
             rt_->launches++;

@@ -95,3 +95,25 @@ def test_large_batch_of_hot_keys_takes_little_memory(kb, rt):
     assert np.array_equal(total, np.bincount(k, v)[key].astype(np.int64)) and np.array_equal(count, np.bincount(k)[key])
     a.close()
     small.close()
+
+
+@pytest.mark.parametrize("expected", [10, 150_000])
+def test_partitioned_batch_in_a_small_budget(kb, rt, expected):
+    """The table holds the keys that there are, not a table's worth for every CTA beside."""
+    budget = 56 << 20
+    small = kb.Runtime.on_torch_stream(0, budget_bytes=budget, stream=rt.torch_stream)
+    rng = np.random.default_rng(expected)
+    n, groups = 300_001, 150_000
+    a = kb.HashAggregate(small, kb.agg_spec(0, [("sum", 1), ("count_star", 0)], expected_groups=expected))
+    ks, vs = [], []
+    for i in range(2):  # the second batch's keys are half known
+        k, v = rng.integers(0, groups, n) + i * groups // 2, rng.integers(-99, 99, n)
+        push(kb, a, k, v)
+        ks.append(k)
+        vs.append(v)
+    k, v = np.concatenate(ks), np.concatenate(vs)
+    key, total, count = groups_of(a)
+    assert np.array_equal(key, np.unique(k))
+    assert np.array_equal(total, np.bincount(k, v)[key].astype(np.int64)) and np.array_equal(count, np.bincount(k)[key])
+    a.close()
+    small.close()
