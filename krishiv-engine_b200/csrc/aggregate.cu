@@ -3157,7 +3157,13 @@ bool HashAggregate::push_few(const DevBatch &b, const KeyIn &key, int64_t n) {
         if (pending_rows_) read_ctl();
         if (known_groups_ + groups + 2 > (int64_t)limit_) grow((uint64_t)known_groups_ + groups + 2);
     }
-    DBuf ovf(rt_, (size_t)n * 4);
+    DBuf ovf;  // room to list every row: without it the batch takes another path
+    try {
+        ovf = DBuf(rt_, (size_t)n * 4);
+    } catch (const Error &e) {
+        if (e.code != KRV_NEED_MEMORY) throw;
+        return false;
+    }
     F.hot_keys = part_hot_keys_.as<long long>();
     F.hot_tab = part_hot_tab_.as<long long>();
     F.hot_tab_idx = part_hot_tab_idx_.as<int16_t>();

@@ -117,3 +117,28 @@ def test_partitioned_batch_in_a_small_budget(kb, rt, expected):
     assert np.array_equal(total, np.bincount(k, v)[key].astype(np.int64)) and np.array_equal(count, np.bincount(k)[key])
     a.close()
     small.close()
+
+
+@pytest.mark.parametrize("keys", [1, 2])
+def test_few_groups_without_room_to_list_the_rows(kb, rt, keys):
+    from test_join_memory_gpu import ballast
+    budget = 256 << 20
+    small = kb.Runtime.on_torch_stream(0, budget_bytes=budget, stream=rt.torch_stream)
+    rng = np.random.default_rng(keys)
+    n = 8_000_003  # 32 MB to list them; 64 MB of codes for two columns
+    k, v = rng.integers(0, 6, n), rng.integers(-99, 99, n)
+    kt = torch.as_tensor(k, device="cuda")
+    cols = [("k", kt, None)] if keys == 1 else [("k0", (kt // 2).to(torch.int32), None), ("k1", (kt % 2).to(torch.int32), None)]
+    cols.append(("v", torch.as_tensor(v, device="cuda"), None))
+    a = kb.HashAggregate(small, kb.agg_spec(0 if keys == 1 else (0, 1), [("sum", keys), ("count_star", 0)], expected_groups=6))
+    b = ballast(kb, small, budget, (16 << 20) if keys == 1 else (110 << 20))
+    a.push_device(kb.DeviceBatch(cols))
+    b.close()
+    a.finish()
+    r = a.result_device()
+    c = [x.cpu().numpy() for x in r.columns]
+    key = c[0] if keys == 1 else c[0].astype(np.int64) * 2 + c[1]
+    assert np.array_equal(np.sort(key), np.arange(6))
+    assert np.array_equal(c[keys], np.bincount(k, v)[key].astype(np.int64)) and np.array_equal(c[keys + 1], np.bincount(k)[key])
+    a.close()
+    small.close()
