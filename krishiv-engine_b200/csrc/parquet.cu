@@ -1556,8 +1556,12 @@ struct BigPlan {
 };
 }  // namespace
 
-ParquetChunk decode_parquet_chunk(Runtime *rt, const uint8_t *chunk, int64_t bytes, const krv_parquet_column &col,
-                                  const KeyFilterImpl *filter) {
+// `device_tables`: large pages of short elements may take the big-page kernels;
+// left true when some did.
+static ParquetChunk decode_chunk(Runtime *rt, const uint8_t *chunk, int64_t bytes, const krv_parquet_column &col,
+                                 const KeyFilterImpl *filter, bool &device_tables) {
+    const bool allow_big = device_tables;
+    device_tables = false;
     if (!chunk && bytes > 0) fail(KRV_INVALID_ARGUMENT, "chunk is NULL");
     if (bytes < 0) fail(KRV_INVALID_ARGUMENT, "chunk_bytes < 0");
     if (col.num_values < 0) fail(KRV_INVALID_ARGUMENT, "num_values < 0");
@@ -1691,7 +1695,7 @@ ParquetChunk decode_parquet_chunk(Runtime *rt, const uint8_t *chunk, int64_t byt
         BigPlan big;
         BigPage bp;
         for (const StageDev &st : stages)
-            if (st.snappy && plan_fragments(chunk, st, frags, true, bp)) big.add(bp);
+            if (st.snappy && plan_fragments(chunk, st, frags, allow_big, bp)) big.add(bp);
         if (!big.pages.empty()) {
             try {
                 big.alloc(rt);
@@ -1704,6 +1708,7 @@ ParquetChunk decode_parquet_chunk(Runtime *rt, const uint8_t *chunk, int64_t byt
                     if (st.snappy) plan_fragments(chunk, st, frags, false, bp);
             }
         }
+        device_tables = !big.pages.empty();
         DBuf dfrags(rt, std::max<size_t>(frags.size(), 1) * sizeof(FragDev));
         if (!frags.empty())
             KRV_CUDA(cudaMemcpyAsync(dfrags.get(), frags.data(), frags.size() * sizeof(FragDev), cudaMemcpyHostToDevice,
@@ -1824,6 +1829,20 @@ ParquetChunk decode_parquet_chunk(Runtime *rt, const uint8_t *chunk, int64_t byt
     r.batch.cols.push_back(out);
     if (filter) r.batch.cols.push_back(pass);
     return r;
+}
+
+ParquetChunk decode_parquet_chunk(Runtime *rt, const uint8_t *chunk, int64_t bytes, const krv_parquet_column &col,
+                                  const KeyFilterImpl *filter) {
+    bool tables = true;
+    try {
+        return decode_chunk(rt, chunk, bytes, col, filter, tables);
+    } catch (const Error &e) {
+        // The big-page kernels' tables are a convenience: a chunk that does not
+        // fit beside them is decoded without.
+        if (e.code != KRV_NEED_MEMORY || !tables) throw;
+    }
+    tables = false;
+    return decode_chunk(rt, chunk, bytes, col, filter, tables);
 }
 
 }  // namespace krv
