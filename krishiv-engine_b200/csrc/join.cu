@@ -1,7 +1,7 @@
 // join.cu -- the hash join operator: build arena, open-addressing table over
-// the engine's key hash, one probe kernel over row tiles whose output is
-// reserved per tile and written with the payload gather fused in, and the
-// right/full join tails.
+// the engine's key hash, a probe in two kernels (the lookup counts every tile's
+// output rows, the emission writes them with the payload gather fused in), and
+// the right/full join tails.
 //
 // Reference: crates/krishiv-exec/src/join/ (HashJoin, join/mod.rs:1014;
 // BuildSink, join/build.rs; ProbeOp, join/probe.rs; JoinIndex,

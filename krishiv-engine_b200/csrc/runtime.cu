@@ -529,7 +529,7 @@ static std::shared_ptr<DBuf> aligned_validity(Runtime *rt, const DevCol &c) {
 void export_host(Runtime *rt, const DevBatch &b, ArrowArray *out, ArrowSchema *out_schema) {
     const size_t n = b.cols.size();
     auto p = std::make_unique<HostArrayPriv>();
-    p->bufs.reserve(2 * n);
+    p->bufs.reserve(3 * n);  // data, string bytes, bitmap: references stay valid
     p->child_bufs.resize(n);
     p->child_storage.resize(n);
     p->children.resize(n);
