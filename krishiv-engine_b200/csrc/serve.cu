@@ -748,8 +748,8 @@ class Server {
         if (opt_.mode == KRV_SERVE_PLAIN) {
             if (!pending_.empty()) {
                 auto r = pending_.front();
-                pending_.pop_front();
                 run_plain(*r);
+                pending_.pop_front();
             }
             return (int64_t)pending_.size();
         }
@@ -888,10 +888,19 @@ class Server {
         while (!pending_.empty() && (int)active_.size() < opt_.max_tick_requests) {
             auto r = pending_.front();
             if (opt_.hbm_budget_bytes > 0 && budget_used_ + (int64_t)r->bytes > opt_.hbm_budget_bytes) break;
-            pending_.pop_front();
             const size_t ng = (size_t)std::max<int64_t>(r->table->ngroups, 1);
-            r->acc = DBuf(rt_, ng * 24);
-            r->out = DBuf(rt_, ng * 24);
+            DBuf acc, out;
+            try {
+                acc = DBuf(rt_, ng * 24);
+                out = DBuf(rt_, ng * 24);
+            } catch (const Error &e) {
+                // the request waits on; those that run may free memory for it
+                if (e.code != KRV_NEED_MEMORY || (active_.empty() && inflight_.empty())) throw;
+                return;
+            }
+            pending_.pop_front();
+            r->acc = std::move(acc);
+            r->out = std::move(out);
             r->admitted = true;
             budget_used_ += (int64_t)r->bytes;
             active_.push_back(r);
