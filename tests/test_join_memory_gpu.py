@@ -122,3 +122,27 @@ def test_probe_with_room_for_little_but_its_output(kb, small, dup, jt, n):
         v = r.columns[2].cpu().numpy()
         assert np.array_equal(k[v % nb], pk[row]) and np.unique(row * (nb * dup) + v).size == out_rows
     j.close()
+
+
+@pytest.mark.parametrize("dup,jt", [(1, "inner"), (3, "inner"), (1, "left_semi"), (1, "left_anti")])
+@pytest.mark.parametrize("n", [1_000_003, 40_003])
+def test_probe_without_room_for_its_lookups(kb, small, dup, jt, n):
+    """Few rows come out: the lookups are what does not fit, and they are made again a chunk at a time."""
+    nb = 5_003
+    k = np.arange(nb) * 1_000_003
+    rng = np.random.default_rng(n + dup)
+    hit = rng.random(n) < (0.99 if jt == "left_anti" else 0.01)
+    pk = np.where(hit, k[rng.integers(0, nb, n)], -1 - np.arange(n))
+    j = kb.HashJoin(small, kb.join_spec(jt, probe_out=[1], build_out=[1] if jt == "inner" else []))
+    j.build_push_device(kb.DeviceBatch([column("k", np.tile(k, dup)), column("v", np.arange(nb * dup))]))
+    j.build_finish()
+    p = kb.DeviceBatch([column("k", pk), column("r", np.arange(n))])
+    b = ballast(kb, small, BUDGET, n * 2 + (64 << 10))
+    r = j.probe_device(p)
+    b.close()
+    out = np.flatnonzero(~hit if jt == "left_anti" else hit)
+    assert np.array_equal(np.sort(r.columns[0].cpu().numpy()), np.repeat(out, dup))
+    if jt == "inner":
+        row, v = (c.cpu().numpy() for c in r.columns)
+        assert np.array_equal(k[v % nb], pk[row]) and np.unique(row * (nb * dup) + v).size == out.size * dup
+    j.close()
