@@ -487,10 +487,74 @@ class GraceJoin {
     void build_push(const DevBatch &in) {
         if (built_) fail(KRV_INVALID_ARGUMENT, "build_push after build_finish");
         DeviceGuard g(rt_);
-        if (!schema_) init_schema(in);
+        if (!schema_) {
+            try {
+                init_schema(in);
+            } catch (...) {  // made anew by the next push
+                build_types_.clear();
+                parts_.clear();
+                bloom_.reset();
+                bloom_bytes_ = 0;
+                throw;
+            }
+        }
         check_shape(in, build_types_, spec_.build_keys[0], "build");
-        counters_.build_rows += in.rows;
-        for (int64_t from = 0; from < in.rows; from += slice_rows()) build_slice(slice(in, from));
+        const Mark m = mark();
+        try {
+            counters_.build_rows += in.rows;
+            for (int64_t from = 0; from < in.rows; from += slice_rows()) build_slice(slice(in, from));
+        } catch (...) {
+            undo(m);
+            throw;
+        }
+    }
+
+    // A batch is taken whole or not at all: what a call that fails in one of
+    // its slices had stored is dropped again, so that the caller may push the
+    // batch once more.
+    struct Mark {
+        struct Side {
+            bool spilled;
+            int64_t build_rows;
+            size_t build_host, probe_host, deferred;
+        };
+        std::vector<Side> parts;
+        size_t pad_later;
+        krv_join_counters counters;
+        int64_t filtered, res_probe_rows, res_out_rows;
+    };
+    Mark mark() const {
+        Mark m{{}, pad_later_.size(), counters_, counters_filtered_, res_probe_rows_, res_out_rows_};
+        for (const Part &P : parts_)
+            m.parts.push_back({P.spilled, P.build_rows, P.build_host.size(), P.probe_host.size(), P.deferred.size()});
+        return m;
+    }
+    void undo(const Mark &m) {
+        for (size_t p = 0; p < parts_.size(); p++) {
+            Part &P = parts_[p];
+            const Mark::Side &was = m.parts[p];
+            P.probe_host.resize(was.probe_host);
+            P.deferred.resize(was.deferred);
+            if (was.spilled) {
+                P.build_host.resize(was.build_host);
+                continue;
+            }
+            if (P.join) P.join->build_truncate(was.build_rows);
+            P.build_rows = was.build_rows;
+            // spilled meanwhile: its arena's rows, in their order, then others
+            int64_t left = was.build_rows;
+            size_t n = 0;
+            for (; n < P.build_host.size() && left > 0; n++) {
+                P.build_host[n].rows = std::min(P.build_host[n].rows, left);
+                left -= P.build_host[n].rows;
+            }
+            P.build_host.resize(n);
+        }
+        pad_later_.resize(m.pad_later);
+        counters_ = m.counters;
+        counters_filtered_ = m.filtered;
+        res_probe_rows_ = m.res_probe_rows;
+        res_out_rows_ = m.res_out_rows;
     }
 
     void build_slice(const DevBatch &b) {
@@ -550,13 +614,19 @@ class GraceJoin {
             check_cols(in, spec_.probe_keys[0], "probe");
         }
         check_shape(in, probe_types_, spec_.probe_keys[0], "probe");
-        counters_.probe_rows += in.rows;
         std::vector<DevBatch> out;
         Share share;
         share.rows_left = in.rows;
         // The batches go out as they are, one per call of krv_join_probe: one
         // batch would cost a copy of them all (and its allocation).
-        for (int64_t from = 0; from < in.rows; from += slice_rows()) probe_slice(slice(in, from), out, share);
+        const Mark m = mark();
+        try {
+            counters_.probe_rows += in.rows;
+            for (int64_t from = 0; from < in.rows; from += slice_rows()) probe_slice(slice(in, from), out, share);
+        } catch (...) {
+            undo(m);
+            throw;
+        }
         KRV_CUDA(cudaStreamSynchronize(rt_->stream));  // the caller's columns are its own again
         return out;
     }

@@ -134,6 +134,8 @@ class HashJoin {
     // Build rows written in place by the caller's kernels.
     void build_reserve(int64_t rows, void **dst);
     void build_commit(int64_t rows);
+    // Takes the rows pushed last back, down to `rows` (before build_finish).
+    void build_truncate(int64_t rows) { build_rows_ = std::min(build_rows_, rows); }
     void build_finish();
     // Joins one probe batch; returns the output batch (all rows of it).
     DevBatch probe(const DevBatch &in);
