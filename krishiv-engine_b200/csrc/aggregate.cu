@@ -2134,6 +2134,7 @@ class HashAggregate {
     void alloc_table(uint64_t slots, DBuf &okeys, DBuf &ogids);
     void unplan();
     void grow(uint64_t need_groups);
+    void grow_to(std::initializer_list<int64_t> groups);
     void launch(const DevBatch &b, const KeyIn &key, int64_t n, const uint32_t *rows_idx, uint32_t *ovf,
                 unsigned long long *ovf_count);
 
@@ -2536,6 +2537,19 @@ void HashAggregate::grow(uint64_t need_groups) {
     rt_->launches++;
     check_launch("rehash_kernel");
     index_pending();
+}
+
+// Grows the table for the first of `groups` that there is memory for (0: for
+// none, it stays as it is).
+void HashAggregate::grow_to(std::initializer_list<int64_t> groups) {
+    for (const int64_t *g = groups.begin(); g != groups.end() && *g; g++) {
+        try {
+            grow((uint64_t)*g);
+            return;
+        } catch (const Error &e) {
+            if (e.code != KRV_NEED_MEMORY || g + 1 == groups.end()) throw;
+        }
+    }
 }
 
 void HashAggregate::index_pending() {
@@ -2997,11 +3011,15 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
         KRV_CUDA(cudaMemsetAsync(start.get(), 0, start.bytes(), rt_->stream));
         // Room in the table for the keys this slice may add (an estimate; a
         // partition that finds none stops and runs again after a grow).
-        // Without a budget there is room for a table's keys of every resident
-        // CTA beside, in case that the estimate is low.
+        // Where there is memory, room for some hundred thousand more beside, in
+        // case that the estimate is low: a growth in the middle of a batch may
+        // find none.
         const int64_t want = known_groups_ + std::min<int64_t>(ns, part_groups_est_) + H + 2;
-        const int64_t beside = rt_->budget == 0 ? (int64_t)part_blocks * rt_->sm_count * fold_cap_ : 0;
-        if (want > (int64_t)limit_ || want + beside > (int64_t)(slots_ / 8 * 7)) grow((uint64_t)(want + beside));
+        const int64_t beside = (int64_t)rt_->sm_count * (rt_->budget == 0 ? part_blocks * fold_cap_ : 2048);
+        if (want > (int64_t)limit_ || want + beside > (int64_t)(slots_ / 8 * 7)) {
+            if (want > (int64_t)limit_) grow_to({want + beside, want});
+            else grow_to({want + beside, 0});
+        }
         const TableDev T = table();
         S.part_buf = part_buf.as<uint8_t>();
         S.part_base = part_base.as<unsigned>();
@@ -3047,7 +3065,8 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
                     again.push_back(p);
                     left += hb[p + 1] - hb[p] - hs[p];
                 }
-            grow((uint64_t)(known_groups_ + std::min<int64_t>(left, (int64_t)again.size() * fold_cap_) + beside + 1));
+            const int64_t need = known_groups_ + std::min<int64_t>(left, (int64_t)again.size() * fold_cap_) + 1;
+            grow_to({need + beside, need, known_groups_ + 1});
             unindexed_from_ = known_groups_;  // grow indexed every group so far
             todo = DBuf(rt_, again.size() * 4);
             KRV_CUDA(cudaMemcpyAsync(todo.get(), again.data(), again.size() * 4, cudaMemcpyHostToDevice, rt_->stream));
