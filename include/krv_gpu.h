@@ -211,7 +211,9 @@ krv_status krv_join_probe_device(krv_join *j, const struct ArrowDeviceArray *in,
                                  struct ArrowDeviceArray *out, struct ArrowSchema *out_schema);
 /* ProbeOp::finish / end_input (join/probe.rs:1149-1228) and emit_build
  * (:610-): rows emitted once every probe row is known (right semi/anti,
- * right/full outer build rows). KRV_HAVE_MORE_OUTPUT or KRV_FINISHED. */
+ * right/full outer build rows). KRV_HAVE_MORE_OUTPUT or KRV_FINISHED. After
+ * KRV_NEED_MEMORY, from here or from a build or probe call, the same call may be
+ * made again: it loses and doubles no rows. */
 krv_status krv_join_finish(krv_join *j, struct ArrowArray *out, struct ArrowSchema *out_schema);
 krv_status krv_join_finish_device(krv_join *j, struct ArrowDeviceArray *out,
                                   struct ArrowSchema *out_schema);
@@ -240,7 +242,7 @@ krv_status krv_hash_rows_device(krv_runtime *rt, const struct ArrowDeviceArray *
  * The engine's grace join (join/grace.rs:828-1481): both sides are radix
  * partitioned by the key hash (level 0: top radix_bits of h, 3..6; a partition
  * still too large is split 8 ways by bits [48-3d, 51-3d) of g); partitions are
- * joined in HBM while their tables fit half of the device budget and spill to
+ * joined in HBM while their tables fit 60% of the device budget and spill to
  * page-locked host memory otherwise. Inner and left outer joins on one int64
  * key (NULL keys allowed); other columns 4 or 8 bytes wide, without NULLs.
  * Same calls as krv_join_*: krv_join_probe returns the rows it can join now
@@ -340,7 +342,9 @@ void krv_agg_spec_init(krv_agg_spec *spec);
 typedef struct krv_agg krv_agg;
 /* HashAggregate::new (aggregate/sink.rs:222) */
 krv_status krv_agg_create(krv_runtime *rt, const krv_agg_spec *spec, krv_agg **out);
-/* HashAggregate::sink (aggregate/sink.rs:1459) */
+/* HashAggregate::sink (aggregate/sink.rs:1459). After KRV_NEED_MEMORY the batch
+ * may be pushed again; when memory ran out with part of its rows taken, that
+ * and every later call returns KRV_INTERNAL instead of wrong sums. */
 krv_status krv_agg_push(krv_agg *a, const struct ArrowArray *batch,
                         const struct ArrowSchema *schema);
 krv_status krv_agg_push_device(krv_agg *a, const struct ArrowDeviceArray *batch,

@@ -2141,6 +2141,13 @@ class HashAggregate {
     Runtime *rt_;
     krv_agg_spec spec_;
     bool planned_ = false, finished_ = false;
+    // From a batch's first update of a record until all its rows are in: a
+    // call that fails between leaves the groups with some of them, and neither
+    // pushing the batch again nor the result would be right then.
+    bool torn_ = false;
+    void check_whole() const {
+        if (torn_) fail(KRV_INTERNAL, "aggregate: a push failed with part of its rows taken");
+    }
     // Group keys other than one int32/int64/date32/decimal(18) column: the
     // dictionary gives each key a dense int64 code, appended to every batch
     // as column key_col_ and aggregated as the key.
@@ -3025,6 +3032,7 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
         S.part_base = part_base.as<unsigned>();
         S.cold = cold;
         const AggPlanDev PS = slice_plan(P, row0, widths);
+        torn_ = true;
         split_kernel<<<S.ctas, kSplitThreads, split_smem, rt_->stream>>>(PS, T, ks, ns, S);
         rt_->launches++;
         check_launch("agg_split_kernel");
@@ -3081,6 +3089,7 @@ void HashAggregate::push_partitioned(const DevBatch &b, const KeyIn &key, int64_
             KRV_CUDA(cudaStreamSynchronize(rt_->stream));  // `again` is a stack vector
         }
     }
+    torn_ = false;
 }
 
 // Undoes plan(), whole or begun.
@@ -3103,6 +3112,7 @@ void HashAggregate::unplan() {
 
 void HashAggregate::push(const DevBatch &in) {
     if (finished_) fail(KRV_INVALID_ARGUMENT, "push after finish");
+    check_whole();
     DeviceGuard g(rt_);
     if (!planned_) {
         try {
@@ -3175,8 +3185,10 @@ void HashAggregate::push(const DevBatch &in) {
     }
     KRV_CUDA(cudaMemsetAsync(&ctl()->deferred, 0, 8, rt_->stream));
     DBuf ovf(rt_, (size_t)n * 4);
+    torn_ = true;
     launch(b, key, n, nullptr, ovf.as<uint32_t>(), &ctl()->deferred);
     run_deferred(b, key, ovf);
+    torn_ = false;
 }
 
 // The batch's rows listed in `ovf` (ctl()->deferred of them), until none is
@@ -3248,11 +3260,13 @@ bool HashAggregate::push_few(const DevBatch &b, const KeyIn &key, int64_t n) {
     int blocks = 0;
     KRV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kFewThreads, smem));
     const int grid = (int)std::min<int64_t>((int64_t)std::max(1, blocks) * rt_->sm_count, ceil_div(n, kFewThreads));
+    torn_ = true;
     kernel<<<grid, kFewThreads, smem, rt_->stream>>>(P, table(), key, n, F);
     rt_->launches++;
     check_launch("agg_few_kernel");
     // a batch of other keys than the sampled ones: later ones are split again
     if (run_deferred(b, key, ovf) > (unsigned long long)n / 16) few_keys_ = false;
+    torn_ = false;
     return true;
 }
 
@@ -3266,6 +3280,7 @@ __global__ void str_code_clean_kernel(long long *codes, const uint8_t *valid, in
 }  // namespace
 
 DevBatch HashAggregate::result() {
+    check_whole();
     DeviceGuard g(rt_);
     DevBatch out;
     if (!planned_) return out;

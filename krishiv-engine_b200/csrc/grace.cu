@@ -13,7 +13,7 @@
 //    of a partition uses bits [48-3d, 51-3d) of g = fin(h ^ seed) (level d,
 //    hash.rs:139-148), 8 ways;
 //  - hybrid residency: partitions are joined in HBM while the build's
-//    estimated footprint (rows, table and chains) fits half of the runtime's
+//    estimated footprint (rows, table and chains) fits 60% of the runtime's
 //    HBM budget; the others spill to page-locked host memory;
 //  - every partition is joined by a HashJoin (the same table, probe and
 //    output code as the unpartitioned join), so the output rows are exactly

@@ -142,3 +142,22 @@ def test_few_groups_without_room_to_list_the_rows(kb, rt, keys):
     assert np.array_equal(c[keys], np.bincount(k, v)[key].astype(np.int64)) and np.array_equal(c[keys + 1], np.bincount(k)[key])
     a.close()
     small.close()
+
+
+def test_a_batch_left_half_taken_is_an_error(kb, rt):
+    """Growth in the middle of a batch finds no memory: no later call gives sums with part of it, or part of it twice."""
+    from test_join_memory_gpu import ballast, status
+    budget = 64 << 20
+    small = kb.Runtime.on_torch_stream(0, budget_bytes=budget, stream=rt.torch_stream)
+    rng = np.random.default_rng(1)
+    k, v = rng.integers(0, 4000, 5000), rng.integers(-9, 9, 5000)
+    a = kb.HashAggregate(small, kb.agg_spec(0, [("sum", 1), ("count_star", 0)], expected_groups=10))
+    push(kb, a, k[:10], v[:10])
+    b = ballast(kb, small, budget, 128 << 10)
+    assert status(kb, push, kb, a, k, v) == kb.NEED_MEMORY
+    b.close()
+    assert status(kb, push, kb, a, k, v) == kb.INTERNAL
+    a.finish()
+    assert status(kb, a.result_device) == kb.INTERNAL
+    a.close()
+    small.close()
