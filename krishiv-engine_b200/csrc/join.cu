@@ -1886,7 +1886,6 @@ DevBatch HashJoin::finish() {
         for (const DevCol &m : out_meta_) empty.cols.push_back(empty_col(m));
         return empty;
     }
-    finished_ = true;
     const bool with_probe = jt == KRV_JOIN_RIGHT_OUTER || jt == KRV_JOIN_FULL_OUTER;
     if (with_probe && probe_types_.empty())
         fail(KRV_INVALID_ARGUMENT, "an outer join's tail needs the probe schema: probe at least one batch");
@@ -1958,6 +1957,7 @@ DevBatch HashJoin::finish() {
         out.cols[v.pos] = var_gather(rt_, src, idx[v.side].as<long long>(), out.rows, m.type, m.nullable, m.name);
     }
     counters_.output_rows += out.rows;
+    finished_ = true;  // only now: a call that failed may be made again
     return out;
 }
 

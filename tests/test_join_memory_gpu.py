@@ -146,3 +146,19 @@ def test_probe_without_room_for_its_lookups(kb, small, dup, jt, n):
         row, v = (c.cpu().numpy() for c in r.columns)
         assert np.array_equal(k[v % nb], pk[row]) and np.unique(row * (nb * dup) + v).size == out.size * dup
     j.close()
+
+
+@pytest.mark.parametrize("jt", ["right_anti", "right_semi", "right_outer", "full_outer"])
+def test_the_tail_comes_when_there_is_memory(kb, small, jt):
+    n = 500_003
+    k = np.arange(n)
+    j = kb.HashJoin(small, kb.join_spec(jt, probe_out=[0], build_out=[1]))
+    j.build_push_device(kb.DeviceBatch([column("k", k), column("v", k * 3)]))
+    j.build_finish()
+    j.probe_device(kb.DeviceBatch([column("k", k[:1000])]))
+    b = ballast(kb, small, BUDGET, 1 << 20)
+    assert status(kb, lambda: list(j.finish_device())) == kb.NEED_MEMORY
+    b.close()
+    v = np.concatenate([r.columns[-1].cpu().numpy() for r in j.finish_device() if r.rows])
+    assert np.array_equal(np.sort(v), k[:1000] * 3 if jt == "right_semi" else k[1000:] * 3)
+    j.close()
